@@ -15,6 +15,8 @@
 
 #include "apsm_common.cuh"
 
+#include <vector>
+
 namespace apsm {
 
 // Settings shared by every job of a batch (one algorithm config).
@@ -26,7 +28,14 @@ struct BatchCommon {
     int XSP;  // pair slots of the sweep's window ring: qP + 3 sp
     int XSPp; // pitch (floats) of the window kernel planes, multiple of 4, >= XSP
     int Np;   // largest complex row pitch of the jobs (float2 units)
+    int cq;   // column n holds entries up to pair n + cq - 1
+    int split; // entries below a pair's window hold the Gaussian part alone (kernels_window_sweep.cu);
+               // 0: every entry is combined (kernels_batch_sweep.cu)
 };
+
+// First combined entry of column n in the split form: the pairs that can still be in the window
+// (or have left it within two steps) when pair n enters.
+__host__ __device__ inline int band_begin(int n, int n_first, int qP) { return n - 1 - qP > n_first ? n - 1 - qP : n_first; }
 
 // One training job: a detector's universe (dictionary pairs already present,
 // then the new pilots) swept by one CTA.
@@ -37,7 +46,7 @@ struct BatchTrainJob {
     float* a;            // 2 nP coefficients (row form); in: old rows, out: visible rows
     float* w;            // 2N linear weights (in/out)
     float* r;            // 2N residual weights r = w - sum_{b visible} a_b x_b (in/out, kept with the detector)
-    const float4* Kc;    // combined kernel columns (A + wL r, Bp + wL m, Bm - wL m, 0), pairs n in [n_first, nP)
+    const float4* Kc;    // kernel columns (A + wL r, Bp + wL m, Bm - wL m, A + wL r), pairs n in [n_first, nP)
     const TrainStep* steps;
     int n_steps;
     int nP, N, Np, capP; // universe pairs, antennas, row pitch (float2), dictionary capacity in pairs
@@ -52,8 +61,22 @@ struct BatchTrainJob {
     // the first window's pairs n < n_first + pro_w (their starting predictions), over
     // b in [col_begin(n), n_first) for the later pairs (the part of their frozen sums whose
     // coefficients this call never changes).
+    // (split form: both ranges end at n_first)
     float2* pro;
     int pro_w, pro_lo, pro_hi, pro_stride;
+    // kernels_window_sweep.cu: sample k of pair b at Yf[b y_pitch + k y_m] (real part) and y_off floats
+    // further (imaginary part); w_init: v starts from w (else from r, which holds it for all pairs but the
+    // last qP of the dictionary); snap_a: the active rows' coefficients after each step (or null)
+    // Its schedule in closed form (window_schedule): pairs visible at the first step, steps of one pass,
+    // whether later passes activate 1, 2, .. pairs.
+    int hi0, t_pass, ramp;
+    const float* Yf;
+    int y_pitch, y_m, y_off;
+    int y_row; // floats of a sample's row to copy (a multiple of 4: 16-byte copies)
+    int nrm_stride; // floats between the norms of consecutive pairs
+    int w_init;
+    float* snap_a;
+    int snap_stride;
 };
 
 // Kernel-column launch shape: columns per block and column entries per pass.
@@ -193,6 +216,19 @@ int batch_sweep_threads();
 cudaError_t batch_sweep_occupancy(const BatchCommon& cm, int* ctas_per_sm);
 cudaError_t launch_batch_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCommon cm, int grid, int* d_counter,
                                int* d_err, cudaStream_t s);
+// The sweep with the window matrix in registers (kernels_window_sweep.cu): one pair per step
+// (sp = 1), windows of up to 93 pairs, dictionaries of at least 2 qP + 2 pairs whose frozen part
+// (at most `range` pairs) fits shared memory beside samples of np antennas.
+// The closed form of a schedule with one pair per step (false: not of that form): first visible end and
+// steps per pass, in pairs; full_start: startWithFullWindow.
+bool window_schedule(const std::vector<TrainStep>& steps, int qP, int capP, bool full_start, int* hi0, int* t_pass);
+bool window_sweep_supports(int qP, int sp, int capP, int range, int np);
+cudaError_t window_sweep_occupancy(const BatchCommon& cm, int range, int* ctas_per_sm);
+cudaError_t launch_window_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCommon cm, int range, int grid,
+                                int* d_counter, int* d_err, cudaStream_t s);
+// Split-form columns [n_first, nP) of the single detector (difference form, kernels_pair_columns.cu).
+cudaError_t launch_pair_columns(const float* X, int N, int Dp, int nP, int n_first, int capP, int qP, float ew,
+                                float wG, float wL, float4* K, cudaStream_t s);
 // Jobs of one antenna class (N <= nmax, nmax in {4, 8, 16, 32, 64}).
 // parts: blocks that share one tile of samples, each taking a contiguous run of
 // the job's 64-pair dictionary chunks (1: one block per tile).  Results do not

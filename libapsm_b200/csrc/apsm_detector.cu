@@ -1,6 +1,7 @@
 // apsm_detector: device state and the train / detect call sequences.
 #include "apsm_host.hpp"
 #include "apsm_kernels.cuh"
+#include "apsm_batch.cuh"
 #include "apsm_gram.cuh"
 #include "apsm_lls.cuh"
 
@@ -251,9 +252,13 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
             span = std::max(span, h_steps[tn].hi - (h_steps[tp].hi - h_steps[tp].wk));
             max_reveal = std::max(max_reveal, h_steps[t].hi - h_steps[t].reveal_lo);
         }
-        APSM_CK(K.ensure(size_t(nV) * Lk));
         APSM_CK(steps.ensure(h_steps.size()));
         APSM_CK(cudaMemcpyAsync(steps.p, h_steps.data(), sizeof(TrainStep) * h_steps.size(), cudaMemcpyHostToDevice, s));
+        if (window_sweep_fits(h_steps, nU)) {
+            APSM_CK(train_window(h_steps, nU, mp, hist_nE > 0, s));
+            goto sweep_done;
+        }
+        APSM_CK(K.ensure(size_t(nV) * Lk));
         {
             dim3 grid((Lk + kGramRows - 1) / kGramRows, (nV + kGramColsPerBlock - 1) / kGramColsPerBlock);
             gram_columns_kernel<<<grid, kGramRows, 0, s>>>(uX.p, int(Dp), int(D), int(nU), v_first, nV, Lk, int(cap),
@@ -448,6 +453,7 @@ sweep_done:
         ha.n_steps = T_steps;
         ha.snap_a = h_snap_a.p;
         ha.snap_w = h_snap_w.p;
+        ha.w0 = window_sweep_fits(h_steps, nU) ? h_w0.p : nullptr;
         ha.snap_scale = cfg.norm_constraint > 0.f ? h_snap_scale.p : nullptr;
         ha.a0 = h_a0.p;
         ha.a0_stride = nU;
@@ -495,6 +501,98 @@ sweep_done:
         APSM_CK(cudaEventElapsedTime(ms, ev0, ev1));
     }
     return APSM_OK;
+}
+
+bool apsm_detector::window_sweep_fits(const std::vector<TrainStep>& h_steps, uint32_t nU) const
+{
+    // normConstraint rescales every coefficient after each step, which the sweep's running predictions do
+    // not follow; APSM_TRAIN_GLOBAL_RING selects a form of the cluster sweep
+    if (cfg.step != 2 || cfg.norm_constraint > 0.f || cfg.train_incremental || force_glob_a) return false;
+    int hi0 = 0, t_pass = 0;
+    return window_sweep_supports(int(cfg.window), 1, int(cap / 2), int(std::min(cap, nU) / 2), int(N)) &&
+           window_schedule(h_steps, int(cfg.window), int(cap / 2), cfg.sfw, &hi0, &t_pass);
+}
+
+// One chain per user over columns that the users share (kernels_window_sweep.cu): one CTA each, 0.35-0.6 us
+// per step against 2.4-3.6 us of the cluster sweep (kernels_sweep.cu), which exchanges the corrections of a
+// window spread over 8 or 16 CTAs and sums every window row over the whole dictionary at each step.
+cudaError_t apsm_detector::train_window(const std::vector<TrainStep>& h_steps, uint32_t nU, const ModelParams& mp,
+                                        bool snapshots, cudaStream_t s)
+{
+    const int qP = int(cfg.window), nP = int(nU / 2), capP = int(cap / 2), T = int(h_steps.size());
+    const int n_first = (h_steps[0].hi - h_steps[0].wk) / 2;
+    const int range = std::min(capP, nP);
+    int hi0 = 0, t_pass = 0;
+    window_schedule(h_steps, qP, capP, cfg.sfw, &hi0, &t_pass);
+    BatchCommon cm{};
+    cm.wL = mp.wL;
+    cm.wG = mp.wG;
+    cm.eB = mp.eB;
+    cm.qP = qP;
+    cm.sp = 1;
+    cm.XSP = qP + 3;
+    cm.Np = int(N);
+    cm.cq = 1;
+    cm.split = 1;
+    const long long base = column_prefix(n_first, 1, nP, capP);
+    cudaError_t e = K.ensure(4 * size_t(column_prefix(nP, 1, nP, capP) - base));
+    if (e != cudaSuccess) return e;
+    e = launch_pair_columns(uX.p, int(N), int(Dp), nP, n_first, capP, qP, mp.ew, mp.wG, mp.wL,
+                            reinterpret_cast<float4*>(K.p), s);
+    if (e != cudaSuccess) return e;
+    if (snapshots) {
+        e = h_w0.ensure(size_t(U) * D);
+        if (e != cudaSuccess) return e;
+        e = cudaMemcpyAsync(h_w0.p, w.p, sizeof(float) * size_t(U) * D, cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) return e;
+    }
+    std::vector<BatchTrainJob> jobs(U);
+    for (uint32_t u = 0; u < U; ++u) {
+        BatchTrainJob& j = jobs[u];
+        j = BatchTrainJob{};
+        j.y = uy.p + size_t(u) * nU;
+        j.a = ua.p + size_t(u) * nU;
+        j.w = w.p + size_t(u) * D;
+        j.Kc = reinterpret_cast<const float4*>(K.p);
+        j.steps = steps.p;
+        j.n_steps = T;
+        j.hi0 = hi0;
+        j.t_pass = t_pass;
+        j.ramp = cfg.sfw ? 0 : 1;
+        j.nP = nP;
+        j.N = int(N);
+        j.capP = capP;
+        j.n_first = n_first;
+        j.used_beforeP = int(used / 2);
+        j.kc_base = base;
+        j.ew = mp.ew;
+        j.nrm = unrm.p;
+        j.nrm_stride = 2; // of the pair's two rows
+        j.Yf = uX.p;
+        j.y_pitch = 2 * int(Dp);
+        j.y_m = 1;
+        j.y_off = int(N);
+        j.y_row = int(Dp);
+        j.w_init = 1;
+        j.snap_a = snapshots ? h_snap_a.p + size_t(u) * T * 2 * qP : nullptr;
+        j.snap_stride = 2 * qP;
+    }
+    e = sweep_jobs.ensure(sizeof(BatchTrainJob) * U + sizeof(int));
+    if (e != cudaSuccess) return e;
+    int* counter = reinterpret_cast<int*>(sweep_jobs.p + sizeof(BatchTrainJob) * U);
+    e = cudaMemcpyAsync(sweep_jobs.p, jobs.data(), sizeof(BatchTrainJob) * U, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counter, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(train_err.p, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaEventRecord(stage_ev[0], s);
+    if (e == cudaSuccess)
+        e = launch_window_sweep(reinterpret_cast<const BatchTrainJob*>(sweep_jobs.p), int(U), cm, range, int(U), counter,
+                                train_err.p, s);
+    if (e == cudaSuccess) e = cudaEventRecord(stage_ev[1], s);
+    stage_valid[0] = true;
+    last_train_cluster = 1;
+    last_train_staged = false;
+    last_train_glob_a = false;
+    return e;
 }
 
 apsm_status apsm_detector::detect(const float2* d_rx, uint32_t S, float2* d_est, cudaStream_t s)

@@ -55,7 +55,9 @@ struct HistoryArgs {
     const TrainStep* steps; // n_steps (the sweep's schedule)
     int n_steps;
     const float* snap_a;    // users x n_steps x q2: active-row coefficients after each step
-    const float* snap_w;    // users x n_steps x D: linear weights after each step
+    float* snap_w;          // users x n_steps x D: linear weights after each step
+    const float* w0;        // users x D: linear weights before the call, for sweeps that leave snap_w to be
+                            // formed from the coefficients (nullptr: snap_w holds the weights)
     const float* snap_scale; // users x n_steps: normConstraint factor of each step (nullptr: none)
     const float* a0;        // users x a0_stride: coefficients of the rows present before the call
     size_t a0_stride;

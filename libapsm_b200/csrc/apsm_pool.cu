@@ -311,6 +311,8 @@ struct apsm_pool {
     struct Schedule {
         std::vector<TrainStep> steps;
         int final_hi = 0;
+        bool regular = false; // of the window sweep's closed form (window_schedule):
+        int hi0 = 0, t_pass = 0;
         long long dev = -1; // offset of its copy in sched_arena (-1: none)
     };
     std::map<std::pair<uint32_t, uint32_t>, Schedule> schedules;
@@ -320,6 +322,7 @@ struct apsm_pool {
         if (it == schedules.end()) {
             Schedule sc;
             sc.steps = build_schedule(cfg, used_before, P, 2 * cfg.dict_size, &sc.final_hi);
+            sc.regular = window_schedule(sc.steps, cm.qP, int(cfg.dict_size), cfg.sfw, &sc.hi0, &sc.t_pass);
             it = schedules.emplace(std::make_pair(used_before, P), std::move(sc)).first;
         }
         return it->second;
@@ -380,6 +383,11 @@ struct apsm_pool {
         return st == APSM_OK ? st : fail(st, what + ": " + msg);
     }
     apsm_status finish(uint32_t lane); // wait for the lane, hand out estimates, check its error flag
+    // training-sweep CTAs per SM for these settings
+    cudaError_t sweep_occupancy(const BatchCommon& c, int* ctas) const
+    {
+        return c.split ? window_sweep_occupancy(c, int(cfg.dict_size), ctas) : batch_sweep_occupancy(c, ctas);
+    }
     apsm_status autotune(uint32_t lane, const apsm_job* jobs, uint32_t n, int mode, std::string* report);
 };
 
@@ -448,6 +456,7 @@ struct TrainPlan {
     const std::vector<TrainStep>* steps = nullptr; // the pool's cached schedule for (rows before, P)
     const void* zc_rx = nullptr; // host-buffer batch: the caller's pilots as the device reads them in place
     const void* zc_tx = nullptr;
+    int hi0 = 0, t_pass = 0; // the schedule's closed form (window sweep)
     long long* steps_dev = nullptr; // its offset in the pool's device schedule arena (-1: not there)
     int final_hi = 0;
     uint32_t P = 0, usedP = 0, nP = 0, n_first = 0;
@@ -566,17 +575,21 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
             t.steps = &sc.steps;
             t.steps_dev = &sc.dev;
             t.final_hi = sc.final_hi;
+            t.hi0 = sc.hi0;
+            t.t_pass = sc.t_pass;
+            if (cm.split && !sc.steps.empty() && !sc.regular)
+                return fail(APSM_ERR_UNSUPPORTED, "training schedule of an unexpected form");
             t.usedP = used0 / 2;
             t.nP = t.usedP + t.P;
             t.n_first = t.steps->empty() ? t.nP : uint32_t((*t.steps)[0].hi - (*t.steps)[0].wk) / 2;
-            t.kc_base = column_prefix(t.n_first, cm.qP, t.nP, t.det->capP);
-            t.n_kc = column_prefix(t.nP, cm.qP, t.nP, t.det->capP) - t.kc_base;
+            t.kc_base = column_prefix(t.n_first, cm.cq, t.nP, t.det->capP);
+            t.n_kc = column_prefix(t.nP, cm.cq, t.nP, t.det->capP) - t.kc_base;
             if (!t.steps->empty() && t.usedP > 0 && !t.fresh) {
                 const int hiP0 = (*t.steps)[0].hi / 2;
                 t.pro_w = hiP0 - int(t.n_first);
                 t.pro_n = int(t.nP - t.n_first);
                 t.pro_lo = std::max(0, hiP0 - int(t.det->capP));
-                t.pro_stride = (int(t.det->capP) + cm.qP + kKcolGroup - 2 + kKcolRows - 1) / kKcolRows + 1;
+                t.pro_stride = (int(t.det->capP) + cm.cq + kKcolGroup - 2 + kKcolRows - 1) / kKcolRows + 1;
             }
             const uint32_t fhP = uint32_t(t.final_hi) / 2;
             t.usedP_new = std::min(fhP, t.det->capP);
@@ -981,8 +994,17 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
         tj.pro = t.pro_n > 0 ? reinterpret_cast<float2*>(D(t.off_pro)) : nullptr;
         tj.pro_w = t.pro_w;
         tj.pro_lo = t.pro_lo;
-        tj.pro_hi = int(t.usedP);
+        tj.pro_hi = cm.split ? int(t.n_first) : int(t.usedP);
         tj.pro_stride = t.pro_stride;
+        tj.Yf = reinterpret_cast<const float*>(Y);
+        tj.y_pitch = 2 * int(d.Np);
+        tj.y_m = 2;
+        tj.y_off = 1;
+        tj.y_row = 2 * int(d.Np);
+        tj.nrm_stride = 1;
+        tj.hi0 = t.hi0;
+        tj.t_pass = t.t_pass;
+        tj.ramp = 1;
         h_tj[k] = tj;
         h_co[k] = BatchCopyJob{Y + size_t(t.lo_new) * d.Np, nrm + t.lo_new, yv + 2 * t.lo_new, av + 2 * t.lo_new,
                                d.Y, d.nrm, d.y, d.a, int(t.usedP_new), int(d.Np)};
@@ -1191,7 +1213,7 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
             // small launches (single train requests): spread each column group's rows over blocks
             int row_split = 1;
             const long long blocks = (long long)kc.count * ((kc.max_cols + batch_kcol_group() - 1) / batch_kcol_group());
-            const int passes = int((int(cfg.dict_size) + cm.qP + batch_kcol_rows() - 1) / batch_kcol_rows());
+            const int passes = int((int(cfg.dict_size) + cm.cq + batch_kcol_rows() - 1) / batch_kcol_rows());
             const long long target = 4LL * std::max(1, sms);
             if (blocks < target)
                 row_split = int(std::min<long long>(std::max(passes, 1), (target + blocks - 1) / blocks));
@@ -1204,7 +1226,8 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
         const int per_sm = shape.sweep_per_sm > 0 ? std::min(shape.sweep_per_sm, sweep_ctas) : sweep_ctas;
         const int grid = int(std::min<size_t>(nT, size_t(per_sm) * sms));
         if (timing) POOL_CK(cudaEventRecord(L.ev[4], s));
-        POOL_CK(launch_batch_sweep(d_tj, int(nT), cm, grid, d_counter, d_err, s));
+        if (cm.split) POOL_CK(launch_window_sweep(d_tj, int(nT), cm, int(cfg.dict_size), grid, d_counter, d_err, s));
+        else POOL_CK(launch_batch_sweep(d_tj, int(nT), cm, grid, d_counter, d_err, s));
         if (timing) POOL_CK(cudaEventRecord(L.ev[5], s));
         if (trace) POOL_CK(cudaEventRecord(L.tr[4], s));
         POOL_CK(launch_batch_copy(reinterpret_cast<const BatchCopyJob*>(D(off_co)), int(nT), max_pairs_out, max_np, s));
@@ -1695,6 +1718,11 @@ extern "C" apsm_status apsm_pool_create(const char* algorithm_json, uint64_t hbm
     cm.LB = cm.qP + cm.sp;
     cm.XSP = cm.qP + 3 * cm.sp;
     cm.XSPp = int(round_up(uint32_t(cm.XSP) + 1, 4));
+    // the sweep with the window matrix in registers, where it holds the configuration (every batch of
+    // the pool then takes it: the form does not depend on what a job is batched with)
+    // (the entering pairs' old-pair sums: at most 64 passes of a column)
+    cm.split = !cfg.sfw && int(cfg.dict_size) <= 62 * kKcolRows && window_sweep_supports(cm.qP, cm.sp, int(cfg.dict_size), int(cfg.dict_size), kMaxFeatures / 2) ? 1 : 0;
+    cm.cq = cm.split ? 1 : cm.qP;
     cm.Np = 32; // sweep shared memory sized for N <= 32; larger N re-sizes at add
     auto failp = [&](const std::string& m, apsm_status st) {
         copy_err(err, errlen, m);
@@ -1755,7 +1783,7 @@ extern "C" apsm_status apsm_pool_create(const char* algorithm_json, uint64_t hbm
     }
     if (cudaStreamCreateWithFlags(&p->sched_stream, cudaStreamNonBlocking) != cudaSuccess)
         return failp("cudaStreamCreate failed", APSM_ERR_CUDA);
-    if (batch_sweep_occupancy(cm, &p->sweep_ctas) != cudaSuccess || p->sweep_ctas < 1)
+    if (p->sweep_occupancy(cm, &p->sweep_ctas) != cudaSuccess || p->sweep_ctas < 1)
         return failp("the training sweep does not fit an SM", APSM_ERR_UNSUPPORTED);
     *out = p;
     return APSM_OK;
@@ -1787,7 +1815,7 @@ extern "C" apsm_status apsm_pool_add(apsm_pool* p, uint32_t num_antennas, uint32
         BatchCommon cm2 = p->cm;
         cm2.Np = int(d.Np);
         int ctas = 0;
-        if (batch_sweep_occupancy(cm2, &ctas) != cudaSuccess || ctas < 1)
+        if (p->sweep_occupancy(cm2, &ctas) != cudaSuccess || ctas < 1)
             return p->fail(APSM_ERR_UNSUPPORTED, "the training sweep does not fit an SM for this antenna count");
         for (auto& l : p->lanes) cudaStreamSynchronize(l.stream);
         p->cm = cm2;

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kColRows)
 {
     // the job's fields in registers: the column stores below cannot alias them then
     const BatchTrainJob& jg = jobs[order ? order[blockIdx.y] : int(blockIdx.y)];
-    const int nP = jg.nP, N = jg.N, Np = jg.Np, capP = jg.capP, qP = cm.qP;
+    const int nP = jg.nP, N = jg.N, Np = jg.Np, capP = jg.capP, cq = cm.cq;
     const int n_first = jg.n_first;
     const int n0 = n_first + blockIdx.x * kColGroup;
     if (n0 >= nP || N > NMAX) return;
@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kColRows)
     // per column: entry range [blo, bhi), store offset of entry b (off + b), old-pair range of its sums
     __shared__ long long s_off[kColGroup];
     __shared__ int s_blo[kColGroup], s_bhi[kColGroup], s_plo[kColGroup], s_phi[kColGroup];
+    __shared__ int s_band[kColGroup]; // first combined entry
 
     if (tid < kColGroup) {
         const int n = n0 + tid;
@@ -60,10 +61,11 @@ __global__ void __launch_bounds__(kColRows)
         long long off = 0;
         if (tid < nc) {
             blo = col_begin(n, capP);
-            bhi = col_end(n, qP, nP);
-            off = column_prefix(n, qP, nP, capP) - jg.kc_base - blo;
+            bhi = col_end(n, cq, nP);
+            off = column_prefix(n, cq, nP, capP) - jg.kc_base - blo;
             if (pro) pro_range(jg, n, &plo, &phi);
         }
+        s_band[tid] = cm.split ? band_begin(n, n_first, cm.qP) : 0;
         s_blo[tid] = blo;
         s_bhi[tid] = bhi;
         s_off[tid] = off;
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(kColRows)
     __syncthreads();
 
     const int b_lo = col_begin(n0, capP); // columns of the group start no earlier
-    const int b_hi = col_end(n0 + nc - 1, qP, nP);
+    const int b_hi = col_end(n0 + nc - 1, cq, nP);
     // grid.z blocks share a column group, each taking every gridDim.z-th pass of rows
     for (int b0 = b_lo + int(blockIdx.z) * kColRows; b0 < b_hi; b0 += int(gridDim.z) * kColRows) {
         // sums over the old pairs (pro_range) of every column, for calls that append
@@ -125,7 +127,9 @@ __global__ void __launch_bounds__(kColRows)
                 const float A = wG * ex2_approx(ewl2 * fmaxf(fmaf(-2.f, re[c], sn), 0.f));
                 const float Bp = wG * ex2_approx(ewl2 * fmaxf(fmaf(-2.f, im[c], sn), 0.f));
                 const float Bm = wG * ex2_approx(ewl2 * fmaxf(fmaf(2.f, im[c], sn), 0.f));
-                const float4 kt = make_float4(fmaf(wL, re[c], A), fmaf(wL, im[c], Bp), fmaf(-wL, im[c], Bm), 0.f);
+                const float wc = b >= s_band[c] ? wL : 0.f;
+                const float4 kt = make_float4(fmaf(wc, re[c], A), fmaf(wc, im[c], Bp), fmaf(-wc, im[c], Bm),
+                                              fmaf(wc, re[c], A));
                 Kc[s_off[c] + b] = kt;
                 if (b >= s_plo[c] && b < s_phi[c]) {
                     // a_2b Kt(2b, .) + a_2b+1 Kt(2b+1, .) for the column pair's two rows

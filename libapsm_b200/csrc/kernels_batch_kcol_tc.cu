@@ -2,7 +2,7 @@
 //
 // Same quantities as batch_kcol_kernel (kernels_batch_kcol.cu): for every pair
 // n entering a window, column n holds against every pair b the sweep combines
-// it with (b in [max(0, n + 1 - capP), min(n + qP, nP))) the combined kernel
+// it with (b in [max(0, n + 1 - capP), min(n + cq, nP))) the combined kernel
 // values (A + wL r, Bp + wL m, Bm - wL m) with r + i m = y_b^H y_n -- the
 // reference's distance loop and linear kernel (cpp/lib/apsm/apsm_detect.cu:
 // 103-152) formed from y_b^H y_n and the pair norms.  The cross terms y_b^H y_n
@@ -106,10 +106,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     const BatchKcolTcJob& jb = jobs[lo];
     const int ci = int(blockIdx.x) - chunk_prefix[lo];
-    const int nP = jb.nP, capP = jb.capP, qP = cm.qP;
+    const int nP = jb.nP, capP = jb.capP, cq = cm.cq;
     const int n0 = jb.n_first + ci * kColPairs;
     const int n_last = min(n0 + kColPairs, nP) - 1;
-    const int b_lo = col_begin(n0, capP), b_hi = col_end(n_last, qP, nP);
+    const int b_lo = col_begin(n0, capP), b_hi = col_end(n_last, cq, nP);
     const int t0 = b_lo / kRowTile, t1 = (b_hi + kRowTile - 1) / kRowTile; // row tiles of the band
     const int ntile = max(0, t1 - t0);
 
@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     float* c_nn = sN + kStages * kRowTile;                // [kColPairs] column norms
     int* c_lo = reinterpret_cast<int*>(c_nn + kColPairs); // [kColPairs] entry range [c_lo, c_hi)
     int* c_hi = c_lo + kColPairs;
-    long long* c_off = reinterpret_cast<long long*>(c_hi + kColPairs); // [kColPairs] store offset of entry 0
+    int* c_band = c_hi + kColPairs;                       // [kColPairs] first combined entry
+    long long* c_off = reinterpret_cast<long long*>(c_band + kColPairs); // [kColPairs] store offset of entry 0
     uint64_t* bars = reinterpret_cast<uint64_t*>(c_off + kColPairs);
     uint64_t* full = bars;              // [kStages]
     uint64_t* empty = bars + kStages;   // [kStages]
@@ -158,12 +159,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         float nv = 0.f;
         if (n < nP) {
             blo = col_begin(n, capP);
-            bhi = col_end(n, qP, nP);
-            off = column_prefix(n, qP, nP, capP) - jb.kc_base - blo;
+            bhi = col_end(n, cq, nP);
+            off = column_prefix(n, cq, nP, capP) - jb.kc_base - blo;
             nv = jb.nrm[n];
         }
         c_lo[threadIdx.x] = blo;
         c_hi[threadIdx.x] = bhi;
+        c_band[threadIdx.x] = cm.split ? band_begin(n, jb.n_first, cm.qP) : 0;
         c_off[threadIdx.x] = off;
         c_nn[threadIdx.x] = nv;
     }
@@ -252,7 +254,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const float A = wG * ex2(ewl2 * fmaxf(fmaf(-2.f, re, sn), 0.f));
                     const float Bp = wG * ex2(ewl2 * fmaxf(fmaf(-2.f, im, sn), 0.f));
                     const float Bm = wG * ex2(ewl2 * fmaxf(fmaf(2.f, im, sn), 0.f));
-                    Kc[c_off[j] + b] = make_float4(fmaf(wL, re, A), fmaf(wL, im, Bp), fmaf(-wL, im, Bm), 0.f);
+                    const float wc = b >= c_band[j] ? wL : 0.f;
+                    const float a = fmaf(wc, re, A);
+                    Kc[c_off[j] + b] = make_float4(a, fmaf(wc, im, Bp), fmaf(-wc, im, Bm), a);
                 }
             }
             tc_fence_before();
@@ -276,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 size_t kcol_tc_smem(int Kpmax)
 {
     return op_bytes(kColN, Kpmax) + size_t(kStages) * op_bytes(kRowTile, Kpmax) + size_t(kStages) * kRowTile * 4 +
-           size_t(kColPairs) * (4 + 4 + 4 + 8) + sizeof(uint64_t) * (2 * kStages + 6) + 16 + 1024;
+           size_t(kColPairs) * (4 + 4 + 4 + 4 + 8) + sizeof(uint64_t) * (2 * kStages + 6) + 16 + 1024;
 }
 
 } // namespace

@@ -70,6 +70,39 @@ __global__ void history_expand_kernel(HistoryArgs h)
     }
 }
 
+// Linear weights of every step from the dense coefficients (HistoryArgs::w0): the change of step t,
+// sum over its active rows of (A[t] - A[t - 1]) x (a row's coefficients before the call at t = 0) ...
+__global__ void __launch_bounds__(kMaxFeatures) history_weight_steps_kernel(HistoryArgs h)
+{
+    const int t = blockIdx.x, u = blockIdx.y, d = threadIdx.x;
+    if (d >= h.D) return;
+    const TrainStep st = h.steps[t];
+    const int start = st.hi - st.wk;
+    const float* A = h.A + (size_t(u) * h.n_steps + t) * h.nU;
+    const float* prev = t > 0 ? A - h.nU : h.a0 + size_t(u) * h.a0_stride;
+    const int n_prev = t > 0 ? h.nU : h.used_before;
+    float acc = 0.f;
+    for (int i = start; i < start + st.n_active; ++i) {
+        const float c = A[i] - (i < n_prev ? prev[i] : 0.f);
+        acc = fmaf(c, h.X[size_t(i) * h.Dp + d], acc);
+    }
+    h.snap_w[(size_t(u) * h.n_steps + t) * h.D + d] = acc;
+}
+
+// ... and their running sums from w0.
+__global__ void __launch_bounds__(kMaxFeatures) history_weight_sum_kernel(HistoryArgs h)
+{
+    const int u = blockIdx.x, d = threadIdx.x;
+    if (d >= h.D) return;
+    float w = h.w0[size_t(u) * h.D + d];
+    float* p = h.snap_w + size_t(u) * h.n_steps * h.D + d;
+#pragma unroll 8
+    for (int t = 0; t < h.n_steps; ++t) {
+        w += p[size_t(t) * h.D];
+        p[size_t(t) * h.D] = w;
+    }
+}
+
 // Shared memory (floats): es[kRows][EP] evaluation rows, xs[kChunk][EP] dictionary
 // rows, kc[kChunk][kRows] kernel values, as[kSteps][kChunk + 1] coefficients,
 // EP = D + 1 (odd pitch: the per-row difference loops are conflict-free).
@@ -235,6 +268,12 @@ cudaError_t launch_history(const HistoryArgs& h, cudaStream_t s)
     history_expand_kernel<<<dim3((h.nU + 255) / 256, h.users), 256, 0, s>>>(h);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    if (h.w0) {
+        history_weight_steps_kernel<<<dim3(h.n_steps, h.users), kMaxFeatures, 0, s>>>(h);
+        history_weight_sum_kernel<<<h.users, kMaxFeatures, 0, s>>>(h);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
     const size_t smem = history_eval_smem(h.D);
     e = cudaFuncSetAttribute(history_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
