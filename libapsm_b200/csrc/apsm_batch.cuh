@@ -64,12 +64,14 @@ struct BatchTrainJob {
     // (split form: both ranges end at n_first)
     float2* pro;
     int pro_w, pro_lo, pro_hi, pro_stride;
+    int pro_passes; // passes of every column (0: those of launch_batch_kcol's column groups)
     // kernels_window_sweep.cu: sample k of pair b at Yf[b y_pitch + k y_m] (real part) and y_off floats
     // further (imaginary part); w_init: v starts from w (else from r, which holds it for all pairs but the
     // last qP of the dictionary); snap_a: the active rows' coefficients after each step (or null)
     // Its schedule in closed form (window_schedule): pairs visible at the first step, steps of one pass,
     // whether later passes activate 1, 2, .. pairs.
     int hi0, t_pass, ramp;
+    int flo; // (the kernel's: first pair of the entering pairs' frozen sums)
     const float* Yf;
     int y_pitch, y_m, y_off;
     int y_row; // floats of a sample's row to copy (a multiple of 4: 16-byte copies)
@@ -229,6 +231,10 @@ cudaError_t launch_window_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCo
 // Split-form columns [n_first, nP) of the single detector (difference form, kernels_pair_columns.cu).
 cudaError_t launch_pair_columns(const float* X, int N, int Dp, int nP, int n_first, int capP, int qP, float ew,
                                 float wG, float wL, float4* K, cudaStream_t s);
+// Sums over the pairs [max(lo_min, first entry), n_first) of those columns, by user: out[user][n - n_first][part],
+// `splits` parts (the window sweep's old-pair sums, BatchTrainJob::pro).
+cudaError_t launch_old_pair_sums(const float4* K, int nP, int n_first, int n_cols, int capP, int lo_min, const float* a,
+                                 size_t a_stride, int users, int splits, float2* out, cudaStream_t s);
 // Jobs of one antenna class (N <= nmax, nmax in {4, 8, 16, 32, 64}).
 // parts: blocks that share one tile of samples, each taking a contiguous run of
 // the job's 64-pair dictionary chunks (1: one block per tile).  Results do not

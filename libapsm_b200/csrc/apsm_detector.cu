@@ -254,8 +254,8 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
         }
         APSM_CK(steps.ensure(h_steps.size()));
         APSM_CK(cudaMemcpyAsync(steps.p, h_steps.data(), sizeof(TrainStep) * h_steps.size(), cudaMemcpyHostToDevice, s));
-        if (window_sweep_fits(h_steps, nU)) {
-            APSM_CK(train_window(h_steps, nU, mp, hist_nE > 0, s));
+        if (const int form = window_sweep_fits(h_steps, nU)) {
+            APSM_CK(train_window(h_steps, nU, mp, hist_nE > 0, form == 2, s));
             goto sweep_done;
         }
         APSM_CK(K.ensure(size_t(nV) * Lk));
@@ -503,25 +503,35 @@ sweep_done:
     return APSM_OK;
 }
 
-bool apsm_detector::window_sweep_fits(const std::vector<TrainStep>& h_steps, uint32_t nU) const
+namespace {
+constexpr int kBlockPairs = 256; // pilots per block of a training call in blocks
+constexpr int kBlockSplits = 4;  // parts of a block's old-pair sums
+} // namespace
+
+// How the window sweep takes a training call: 1 one launch; 2 in blocks of kBlockPairs pilots (dictionaries
+// whose frozen sums do not fit its shared memory: above 2729 pairs); 0 not at all (the cluster sweep).
+int apsm_detector::window_sweep_fits(const std::vector<TrainStep>& h_steps, uint32_t nU) const
 {
     // normConstraint rescales every coefficient after each step, which the sweep's running predictions do
     // not follow; APSM_TRAIN_GLOBAL_RING selects a form of the cluster sweep
-    if (cfg.step != 2 || cfg.norm_constraint > 0.f || cfg.train_incremental || force_glob_a) return false;
+    if (cfg.step != 2 || cfg.norm_constraint > 0.f || cfg.train_incremental || force_glob_a) return 0;
     int hi0 = 0, t_pass = 0;
-    return window_sweep_supports(int(cfg.window), 1, int(cap / 2), int(std::min(cap, nU) / 2), int(N)) &&
-           window_schedule(h_steps, int(cfg.window), int(cap / 2), cfg.sfw, &hi0, &t_pass);
+    const int qP = int(cfg.window), capP = int(cap / 2), range = int(std::min(cap, nU) / 2);
+    if (!window_schedule(h_steps, qP, capP, cfg.sfw, &hi0, &t_pass)) return 0;
+    if (window_sweep_supports(qP, 1, capP, range, int(N))) return 1;
+    if (cfg.passes == 1 && !cfg.sfw && window_sweep_supports(qP, 1, capP, kBlockPairs + 2 * qP, int(N))) return 2;
+    return 0;
 }
 
-// One chain per user over columns that the users share (kernels_window_sweep.cu): one CTA each, 0.35-0.6 us
-// per step against 2.4-3.6 us of the cluster sweep (kernels_sweep.cu), which exchanges the corrections of a
-// window spread over 8 or 16 CTAs and sums every window row over the whole dictionary at each step.
+// One chain per user over columns that the users share (kernels_window_sweep.cu), one CTA each: about 1 us a
+// step at window 80 against 2.4-3.6 us of the cluster sweep (kernels_sweep.cu; 84 us with 8192 pilots of 64
+// antennas and 16 users), which exchanges the corrections of a window spread over 8 or 16 CTAs and sums every
+// window row over the whole dictionary at each step.  In blocks, each block is an appending call to the pairs
+// before it: its columns, their sums over those pairs for every user (one launch over all SMs), its sweep.
 cudaError_t apsm_detector::train_window(const std::vector<TrainStep>& h_steps, uint32_t nU, const ModelParams& mp,
-                                        bool snapshots, cudaStream_t s)
+                                        bool snapshots, bool blocks, cudaStream_t s)
 {
-    const int qP = int(cfg.window), nP = int(nU / 2), capP = int(cap / 2), T = int(h_steps.size());
-    const int n_first = (h_steps[0].hi - h_steps[0].wk) / 2;
-    const int range = std::min(capP, nP);
+    const int qP = int(cfg.window), capP = int(cap / 2), T = int(h_steps.size());
     int hi0 = 0, t_pass = 0;
     window_schedule(h_steps, qP, capP, cfg.sfw, &hi0, &t_pass);
     BatchCommon cm{};
@@ -534,59 +544,99 @@ cudaError_t apsm_detector::train_window(const std::vector<TrainStep>& h_steps, u
     cm.Np = int(N);
     cm.cq = 1;
     cm.split = 1;
-    const long long base = column_prefix(n_first, 1, nP, capP);
-    cudaError_t e = K.ensure(4 * size_t(column_prefix(nP, 1, nP, capP) - base));
+    struct Block {
+        int hi0, t0, t_pass, n_steps, nP, n_first, used;
+    };
+    std::vector<Block> list;
+    for (int t0 = 0; t0 < t_pass; t0 += kBlockPairs) {
+        Block b;
+        b.hi0 = hi0 + t0;
+        b.t0 = t0;
+        b.t_pass = blocks ? std::min(kBlockPairs, t_pass - t0) : t_pass;
+        b.n_steps = blocks ? b.t_pass : T;
+        b.nP = blocks ? b.hi0 + b.t_pass - 1 : int(nU / 2);
+        b.n_first = std::max(0, b.hi0 - qP);
+        b.used = t0 == 0 ? int(used / 2) : b.hi0 - 1;
+        list.push_back(b);
+        if (!blocks) break;
+    }
+    size_t columns = 0, sums = 0;
+    for (const Block& b : list) {
+        columns = std::max(columns, size_t(column_prefix(b.nP, 1, b.nP, capP) - column_prefix(b.n_first, 1, b.nP, capP)));
+        if (b.used > 0 && blocks) sums = std::max(sums, size_t(U) * (b.nP - b.n_first) * kBlockSplits);
+    }
+    cudaError_t e = K.ensure(4 * columns);
     if (e != cudaSuccess) return e;
-    e = launch_pair_columns(uX.p, int(N), int(Dp), nP, n_first, capP, qP, mp.ew, mp.wG, mp.wL,
-                            reinterpret_cast<float4*>(K.p), s);
-    if (e != cudaSuccess) return e;
+    if (sums > 0) {
+        e = sweep_sums.ensure(2 * sums);
+        if (e == cudaSuccess) e = sweep_v.ensure(size_t(U) * D);
+        if (e != cudaSuccess) return e;
+    }
     if (snapshots) {
         e = h_w0.ensure(size_t(U) * D);
-        if (e != cudaSuccess) return e;
-        e = cudaMemcpyAsync(h_w0.p, w.p, sizeof(float) * size_t(U) * D, cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(h_w0.p, w.p, sizeof(float) * size_t(U) * D, cudaMemcpyDeviceToDevice, s);
         if (e != cudaSuccess) return e;
     }
-    std::vector<BatchTrainJob> jobs(U);
-    for (uint32_t u = 0; u < U; ++u) {
-        BatchTrainJob& j = jobs[u];
-        j = BatchTrainJob{};
-        j.y = uy.p + size_t(u) * nU;
-        j.a = ua.p + size_t(u) * nU;
-        j.w = w.p + size_t(u) * D;
-        j.Kc = reinterpret_cast<const float4*>(K.p);
-        j.steps = steps.p;
-        j.n_steps = T;
-        j.hi0 = hi0;
-        j.t_pass = t_pass;
-        j.ramp = cfg.sfw ? 0 : 1;
-        j.nP = nP;
-        j.N = int(N);
-        j.capP = capP;
-        j.n_first = n_first;
-        j.used_beforeP = int(used / 2);
-        j.kc_base = base;
-        j.ew = mp.ew;
-        j.nrm = unrm.p;
-        j.nrm_stride = 2; // of the pair's two rows
-        j.Yf = uX.p;
-        j.y_pitch = 2 * int(Dp);
-        j.y_m = 1;
-        j.y_off = int(N);
-        j.y_row = int(Dp);
-        j.w_init = 1;
-        j.snap_a = snapshots ? h_snap_a.p + size_t(u) * T * 2 * qP : nullptr;
-        j.snap_stride = 2 * qP;
-    }
-    e = sweep_jobs.ensure(sizeof(BatchTrainJob) * U + sizeof(int));
+    std::vector<BatchTrainJob> jobs(list.size() * U);
+    for (size_t i = 0; i < list.size(); ++i)
+        for (uint32_t u = 0; u < U; ++u) {
+            const Block& b = list[i];
+            BatchTrainJob& j = jobs[i * U + u];
+            j = BatchTrainJob{};
+            j.y = uy.p + size_t(u) * nU;
+            j.a = ua.p + size_t(u) * nU;
+            j.w = w.p + size_t(u) * D;
+            j.r = blocks && sweep_v.p ? sweep_v.p + size_t(u) * D : nullptr;
+            j.Kc = reinterpret_cast<const float4*>(K.p);
+            j.steps = steps.p;
+            j.n_steps = b.n_steps;
+            j.hi0 = b.hi0;
+            j.t_pass = b.t_pass;
+            j.ramp = cfg.sfw ? 0 : 1;
+            j.nP = b.nP;
+            j.N = int(N);
+            j.capP = capP;
+            j.n_first = b.n_first;
+            j.used_beforeP = b.used;
+            j.kc_base = column_prefix(b.n_first, 1, b.nP, capP);
+            j.ew = mp.ew;
+            j.nrm = unrm.p;
+            j.nrm_stride = 2; // of the pair's two rows
+            j.Yf = uX.p;
+            j.y_pitch = 2 * int(Dp);
+            j.y_m = 1;
+            j.y_off = int(N);
+            j.y_row = int(Dp);
+            j.w_init = b.t0 == 0 ? 1 : 0;
+            if (blocks && b.used > 0) {
+                j.pro = reinterpret_cast<float2*>(sweep_sums.p) + size_t(u) * (b.nP - b.n_first) * kBlockSplits;
+                j.pro_stride = j.pro_passes = kBlockSplits;
+            }
+            j.snap_a = snapshots ? h_snap_a.p + (size_t(u) * T + b.t0) * 2 * qP : nullptr;
+            j.snap_stride = 2 * qP;
+        }
+    const size_t job_bytes = sizeof(BatchTrainJob) * jobs.size();
+    e = sweep_jobs.ensure(job_bytes + sizeof(int) * list.size());
     if (e != cudaSuccess) return e;
-    int* counter = reinterpret_cast<int*>(sweep_jobs.p + sizeof(BatchTrainJob) * U);
-    e = cudaMemcpyAsync(sweep_jobs.p, jobs.data(), sizeof(BatchTrainJob) * U, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(counter, 0, sizeof(int), s);
+    int* counters = reinterpret_cast<int*>(sweep_jobs.p + job_bytes);
+    e = cudaMemcpyAsync(sweep_jobs.p, jobs.data(), job_bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, sizeof(int) * list.size(), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(train_err.p, 0, sizeof(int), s);
     if (e == cudaSuccess) e = cudaEventRecord(stage_ev[0], s);
-    if (e == cudaSuccess)
-        e = launch_window_sweep(reinterpret_cast<const BatchTrainJob*>(sweep_jobs.p), int(U), cm, range, int(U), counter,
-                                train_err.p, s);
+    for (size_t i = 0; i < list.size() && e == cudaSuccess; ++i) {
+        const Block& b = list[i];
+        const BatchTrainJob& j = jobs[i * U];
+        e = launch_pair_columns(uX.p, int(N), int(Dp), b.nP, b.n_first, capP, qP, mp.ew, mp.wG, mp.wL,
+                                reinterpret_cast<float4*>(K.p), s);
+        if (e == cudaSuccess && j.pro)
+            e = launch_old_pair_sums(j.Kc, b.nP, b.n_first, b.nP - b.n_first, capP, std::max(0, b.hi0 - capP), ua.p, nU, int(U), kBlockSplits,
+                                     reinterpret_cast<float2*>(sweep_sums.p), s);
+        const int range = blocks ? kBlockPairs + 2 * qP : std::min(capP, b.nP);
+        if (e == cudaSuccess)
+            e = launch_window_sweep(reinterpret_cast<const BatchTrainJob*>(sweep_jobs.p) + i * U, int(U), cm, range, int(U),
+                                    counters + i, train_err.p, s);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(stage_ev[1], s);
     stage_valid[0] = true;
     last_train_cluster = 1;

@@ -102,6 +102,7 @@ struct apsm_detector {
     // per-call scratch
     apsm::DevBuf<float> uX, unrm, uy, ua, K, xs;
     apsm::DevBuf<uint8_t> sweep_jobs; // window sweep: the users' job descriptors and the job counter
+    apsm::DevBuf<float> sweep_sums, sweep_v; // and, in blocks, the old-pair sums and the residual weights
     apsm::DevBuf<float> a_rings; // exact sweep: per-CTA coefficient rings of large dictionaries
     apsm::DevBuf<apsm::TrainStep> steps;
     apsm::DevBuf<int> train_err; // set by the sweep when a bounded wait expired
@@ -132,9 +133,9 @@ struct apsm_detector {
     apsm_status reset();
     apsm_status train(const float2* d_rx, const float2* d_tx, uint32_t P, cudaStream_t s, float* ms,
                       apsm::HistoryRequest* hist = nullptr);
-    bool window_sweep_fits(const std::vector<apsm::TrainStep>& h_steps, uint32_t nU) const;
+    int window_sweep_fits(const std::vector<apsm::TrainStep>& h_steps, uint32_t nU) const;
     cudaError_t train_window(const std::vector<apsm::TrainStep>& h_steps, uint32_t nU, const apsm::ModelParams& mp,
-                             bool snapshots, cudaStream_t s);
+                             bool snapshots, bool blocks, cudaStream_t s);
     apsm_status train_history_host(const float2* rx, const float2* tx, uint32_t P, const float2* rx_val,
                                    const float2* tx_val, uint32_t S, uint32_t bps, float mod_scale, float* history,
                                    uint32_t max_steps, uint32_t* n_steps, float* ms);

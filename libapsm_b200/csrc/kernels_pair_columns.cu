@@ -155,7 +155,84 @@ __global__ void __launch_bounds__(256, 2) pair_columns_kernel(PairColumnsArgs g)
     else columns_tile<false>(g, b0, n0, sb, sn);
 }
 
+// Old-pair sums of columns [n_first, n_first + n_cols) for every user: sum over the pairs b < n_first
+// that pair n meets (b >= lo_min: visible at the call's first step) of a_b K(b, n), in `splits` parts ([user][n - n_first][part]).  A block takes kSumCols
+// columns x kSumUsers users x one part of the pairs: 128 fma per 12 loads of a thread, the columns
+// (from DRAM) read once for 8 users, the coefficients (from L2) once for 4 columns.
+constexpr int kSumCols = 4, kSumUsers = 8, kSumThreads = 128;
+
+__global__ void __launch_bounds__(kSumThreads)
+    old_pair_sums_kernel(const float4* __restrict__ K, long long base, int nP, int n_first, int n_cols, int capP, int lo_min,
+                         const float* __restrict__ a, size_t a_stride, int users, int splits, float2* __restrict__ out)
+{
+    __shared__ float2 part[kSumThreads / 32][kSumCols * kSumUsers];
+    const int c0 = blockIdx.x * kSumCols, u0 = blockIdx.y * kSumUsers, sp = blockIdx.z;
+    const float4* col[kSumCols];
+    int lo[kSumCols];
+#pragma unroll
+    for (int c = 0; c < kSumCols; ++c) {
+        const int n = n_first + min(c0 + c, n_cols - 1);
+        lo[c] = max(col_begin(n, capP), lo_min);
+        col[c] = K + (column_prefix(n, 1, nP, capP) - base) - col_begin(n, capP);
+    }
+    float2 g[kSumCols][kSumUsers];
+#pragma unroll
+    for (int c = 0; c < kSumCols; ++c)
+#pragma unroll
+        for (int u = 0; u < kSumUsers; ++u) g[c][u] = make_float2(0.f, 0.f);
+    const int len = (n_first - lo[0] + splits - 1) / splits;
+    const int b_end = min(n_first, lo[0] + (sp + 1) * len);
+    for (int b = lo[0] + sp * len + int(threadIdx.x); b < b_end; b += kSumThreads) {
+        float4 k[kSumCols];
+#pragma unroll
+        for (int c = 0; c < kSumCols; ++c) k[c] = b >= lo[c] ? __ldg(col[c] + b) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < kSumUsers; ++u) {
+            const float2 ab = u0 + u < users ? *reinterpret_cast<const float2*>(a + size_t(u0 + u) * a_stride + 2 * b)
+                                             : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < kSumCols; ++c) {
+                g[c][u].x = fmaf(ab.x, k[c].x, fmaf(ab.y, k[c].z, g[c][u].x));
+                g[c][u].y = fmaf(ab.x, k[c].y, fmaf(ab.y, k[c].x, g[c][u].y));
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < kSumCols; ++c)
+#pragma unroll
+        for (int u = 0; u < kSumUsers; ++u) {
+            float2 v = g[c][u];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+                v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+            }
+            if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][c * kSumUsers + u] = v;
+        }
+    __syncthreads();
+    if (threadIdx.x < kSumCols * kSumUsers) {
+        const int c = threadIdx.x / kSumUsers, u = threadIdx.x % kSumUsers;
+        float2 v = part[0][threadIdx.x];
+#pragma unroll
+        for (int w = 1; w < kSumThreads / 32; ++w) {
+            v.x += part[w][threadIdx.x].x;
+            v.y += part[w][threadIdx.x].y;
+        }
+        if (c0 + c < n_cols && u0 + u < users) out[(size_t(u0 + u) * n_cols + c0 + c) * splits + sp] = v;
+    }
+}
+
 } // namespace
+
+cudaError_t launch_old_pair_sums(const float4* K, int nP, int n_first, int n_cols, int capP, int lo_min, const float* a,
+                                 size_t a_stride, int users, int splits, float2* out, cudaStream_t s)
+{
+    if (n_cols <= 0) return cudaSuccess;
+    old_pair_sums_kernel<<<dim3((n_cols + kSumCols - 1) / kSumCols, (users + kSumUsers - 1) / kSumUsers, splits),
+                           kSumThreads, 0, s>>>(K, column_prefix(n_first, 1, nP, capP), nP, n_first, n_cols, capP,
+                                                lo_min, a, a_stride, users, splits, out);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_pair_columns(const float* X, int N, int Dp, int nP, int n_first, int capP, int qP, float ew,
                                 float wG, float wL, float4* K, cudaStream_t s)

@@ -62,6 +62,7 @@ template <int C_, int RG_, int TR_, int BLOCKS_> struct Shape {
     static constexpr int kThreads = 32 * (kHelpWarps + RG);
     static constexpr int kCols = 32 * C;                       // pair slots (columns)
     static constexpr int kSlots = kCols > RG * TR ? kCols : RG * TR;
+    static constexpr int kMatrix = C == 1 ? 1024 : (C == 2 ? 4096 : 8192); // RG TR x kCols entries, a power of two
     static constexpr int kRed = RG * 2 * kCols > kHelpWarps * kMaxFeatures ? RG * 2 * kCols : kHelpWarps * kMaxFeatures;
 };
 
@@ -71,12 +72,29 @@ struct Layout {
     int pitch;  // floats per sample
 };
 
+// Shared memory: the parts of fixed size first (their addresses are constants), then stream, ring
+// and samples.
+template <class S> struct alignas(128) Shared {
+    float4 nbuf[S::kSlots];                      // entering pair's column by slot
+    float4 evk[kEvictAhead * kRowThreads];       // evicted pair's entries by row thread
+    float4 rec[64];                              // entering pairs: y0, y1, projection scale, by te
+    float2 eva[kEvictAhead * kRowThreads];       // evicted pair's coefficients
+    float2 cs[S::kSlots];                        // corrections by slot
+    float2 aw[2 * S::kSlots];                    // window coefficients by step parity
+    float2 prs[64];                              // old-pair sums of the entering pairs, by te
+    float2 lp[4 * 32];                           // warp kPrepWarp's share of the starts, by te
+    float red[S::kRed];                          // [RG][2 kCols] update partials
+    float hw[2 * S::kSlots];                     // first predictions
+    float vs[kMaxFeatures];
+    uint64_t cfull[kGroups], xfull[2];           // column and sample groups have arrived
+    BatchTrainJob js;
+    int abort_flag, stop[2], job;                // stop: the abort flag as every thread of a step sees it
+    uint32_t base[2];                            // column and sample groups of the jobs before (phases run on)
+};
+
 template <class S> __host__ __device__ inline size_t smem_bytes(const Layout& l)
 {
-    return 16 * (size_t(l.stream) + S::kSlots + size_t(kEvictAhead) * kRowThreads + 64) +
-           8 * (size_t(l.ring) + size_t(kEvictAhead) * kRowThreads + 3 * S::kSlots + 64) +
-           4 * (size_t(4) * kSampleBatch * l.pitch + S::kRed + 4 * S::kSlots + kMaxFeatures + 32) +
-           8 * (kGroups + 2) + 64;
+    return sizeof(Shared<S>) + 16 * size_t(l.stream) + 8 * size_t(l.ring) + 4 * size_t(4) * kSampleBatch * l.pitch + 128;
 }
 
 // apsm_train.cu:380-401, without branches (a divergent branch costs the chain some 50 cycles)
@@ -168,19 +186,20 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
     return d;
 }
 
-// Register updates of the tile in place, predicated (selects on the register arrays made the compiler copy
-// the whole tile every step).
-__device__ __forceinline__ void set_if(f32x2& x, f32x2& y, f32x2 nx, f32x2 ny, int a, int b)
+// Register updates of the tile in place (selects on the register arrays made the compiler copy the whole tile
+// several times a step).
+__device__ __forceinline__ void set(float& a, float& p, float& m, float na, float np, float nm)
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %4, %5;\n\t@p mov.b64 %0, %2;\n\t@p mov.b64 %1, %3;\n\t}"
-                 : "+l"(x), "+l"(y)
-                 : "l"(nx), "l"(ny), "r"(a), "r"(b));
+    asm volatile("mov.b32 %0, %3;\n\tmov.b32 %1, %4;\n\tmov.b32 %2, %5;"
+                 : "+f"(a), "+f"(p), "+f"(m)
+                 : "f"(na), "f"(np), "f"(nm));
 }
-__device__ __forceinline__ void load_if(f32x2& x, f32x2& y, uint32_t addr, int a, int b)
+__device__ __forceinline__ void load_if(float& a, float& p, float& m, uint32_t addr, int pred)
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %3, %4;\n\t@p ld.shared.v2.b64 {%0, %1}, [%2];\n\t}"
-                 : "+l"(x), "+l"(y)
-                 : "r"(addr), "r"(a), "r"(b)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %4, 0;\n\t@q ld.shared.v2.f32 {%0, %1}, [%3];\n\t"
+                 "@q ld.shared.f32 %2, [%3 + 8];\n\t}"
+                 : "+f"(a), "+f"(p), "+f"(m)
+                 : "r"(addr), "r"(pred)
                  : "memory");
 }
 
@@ -238,10 +257,11 @@ struct JobView {
     }
     // frozen range [frozen_lo, frozen_hi) of the pair n entering the window
     __device__ __forceinline__ int frozen_hi(int n) const { return band_begin(n, n_first, qP); }
-    __device__ __forceinline__ int frozen_lo(int n) const { return max(col_begin(n, capP), pro ? n_first : 0); }
+    __device__ __forceinline__ int frozen_lo(int n) const { return max(col_begin(n, capP), j.flo); }
     // sums of the old pairs [.., n_first) of column n that the kernel-column launch formed, one per pass
     __device__ __forceinline__ int pro_passes(int n) const
     {
+        if (j.pro_passes > 0) return j.pro_passes;
         const int g0 = n_first + (n - n_first) / kKcolGroup * kKcolGroup;
         const int gl = min(g0 + kKcolGroup, nP) - 1;
         return (col_end(gl, 1, nP) - col_begin(g0, capP) + kKcolRows - 1) / kKcolRows;
@@ -256,29 +276,18 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
     constexpr int C = S::C, RG = S::RG, TR = S::TR, kCols = S::kCols, kSlots = S::kSlots;
     constexpr int kAll = S::kThreads, kSampleGroups = 2;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    float4* stream = reinterpret_cast<float4*>(smem_raw);         // [lay.stream] columns of the entering pairs
+    Shared<S>& m = *reinterpret_cast<Shared<S>*>(smem_raw);
+    float4* const stream = reinterpret_cast<float4*>(smem_raw + sizeof(Shared<S>)); // columns of the entering pairs
+    float2* const ring = reinterpret_cast<float2*>(stream + lay.stream); // coefficients, pair b at b mod ring
     // [2 kSampleBatch][2][lay.pitch] samples of the entering pairs and of those that join v with them, by te
-    float* xs = reinterpret_cast<float*>(stream + lay.stream);
-    float4* nbuf = reinterpret_cast<float4*>(xs + size_t(4) * kSampleBatch * lay.pitch); // [kSlots] entering pair's column by slot
-    float4* evk = nbuf + kSlots;                                  // [kEvictAhead][kRowThreads] evicted pair's entries
-    float4* rec = evk + kEvictAhead * kRowThreads;                // [64] entering pairs: y0, y1, projection scale, by te
-    float2* eva = reinterpret_cast<float2*>(rec + 64);            // [kEvictAhead][kRowThreads] and coefficients
-    float2* ring = eva + kEvictAhead * kRowThreads;               // coefficients, pair b at b mod ring
-    float2* cs = ring + lay.ring;                                 // [kSlots] corrections by slot
-    float2* prs = cs + kSlots;                                    // [64] old-pair sums of the entering pairs, by te
-    float2* aw = prs + 64;                                        // [2][kSlots] window coefficients by step parity
-    float* red = reinterpret_cast<float*>(aw + 2 * kSlots);       // [RG][2 kCols] update partials
-    float* hw = red + S::kRed;                                    // [2 kSlots] first predictions
-    float* vs = hw + 4 * kSlots;                                  // [kMaxFeatures]
-    float* st = vs + kMaxFeatures;                                // [4][2] linear and old-pair part of an entering pair's start, by te
-    uint64_t* cfull = reinterpret_cast<uint64_t*>(st + 32);       // [kGroups] columns
-    uint64_t* xfull = cfull + kGroups;                            // [kSampleGroups] samples
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(xfull + kSampleGroups);
-    volatile int* stop = abort_flag + 1; // [2] the abort flag as every thread of a step sees it
-    volatile int* job_s = abort_flag + 3;
-    volatile uint32_t* base_s = reinterpret_cast<volatile uint32_t*>(abort_flag + 4); // [2] column and sample groups of
-                                                                                      // the jobs before (phases run on)
-    __shared__ BatchTrainJob js;
+    float* const xs = reinterpret_cast<float*>(ring + lay.ring);
+    float4 *const nbuf = m.nbuf, *const evk = m.evk, *const rec = m.rec;
+    float2 *const eva = m.eva, *const cs = m.cs, *const aw = m.aw, *const prs = m.prs, *const lp = m.lp;
+    float *const red = m.red, *const hw = m.hw, *const vs = m.vs;
+    uint64_t *const cfull = m.cfull, *const xfull = m.xfull;
+    volatile int *const abort_flag = &m.abort_flag, *const stop = m.stop, *const job_s = &m.job;
+    volatile uint32_t* const base_s = m.base;
+    BatchTrainJob& js = m.js;
     const uint32_t smask = uint32_t(lay.stream) - 1, rmask = uint32_t(lay.ring) - 1;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -294,14 +303,17 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
 
-    // (A, Bp) and (Bm, A) of row slots cw TR + k against pair slots lane + 32 j, at j TR + k
-    f32x2 tX[TR * C], tY[TR * C];
+    // (A, Bp, Bm) of row slots cw TR + k against pair slots lane + 32 j, at j TR + k
+    float tA[TR * C], tP[TR * C], tM[TR * C];
 
     for (;;) {
         __syncthreads();
         if (tid == 0) {
             *job_s = atomicAdd(counter, 1);
-            if (*job_s < n_jobs) js = jobs[*job_s];
+            if (*job_s < n_jobs) {
+                js = jobs[*job_s];
+                js.flo = js.pro ? js.n_first : 0;
+            }
         }
         for (int i = tid; i < S::kRed; i += S::kThreads) red[i] = 0.f;
         for (int i = tid; i < kSlots; i += S::kThreads) cs[i] = aw[i] = aw[kSlots + i] = make_float2(0.f, 0.f);
@@ -363,23 +375,32 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                 warp_sum2(g0, g1);
                 if (lane == 0) *reinterpret_cast<float2*>(hw + 2 * v.slot_of(j)) = make_float2(g0, g1);
             }
-        // the window's kernel matrix
-        if (cw >= 0) {
-#pragma unroll
-            for (int i = 0; i < TR * C; ++i) {
-                const int q = 32 * (i / TR) + lane, jq = v.pair_of_slot(q, s0, los0);
-                const int p = cw * TR + i % TR, bp = v.pair_of_slot(p, s0, los0);
-                tX[i] = tY[i] = 0ull;
-                if (q < v.RP && p < v.RP && jq < hi0 && bp < hi0) {
-                    const ulonglong2 kv = __ldg(reinterpret_cast<const ulonglong2*>(v.col_ptr(max(jq, bp)) + min(jq, bp)));
-                    const float2 x = unpack2(kv.x), y = unpack2(kv.y); // (A, Bp), (Bm, A); transposed: Bp, Bm swapped
-                    tX[i] = bp <= jq ? kv.x : pack2(x.x, y.x);
-                    tY[i] = bp <= jq ? kv.y : pack2(x.y, y.y);
-                }
+        // the window's kernel matrix, by slots in the stream buffer (rows of kCols), then into the tile
+        for (int i = tid; i < RG * TR * kCols; i += S::kThreads) stream[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        for (int j = s0 + warp; j < hi0; j += S::kThreads / 32) {
+            const float4* col = v.col_ptr(j);
+            const int sj = v.slot_of(j);
+            for (int b = s0 + lane; b <= j; b += 32) {
+                const float4 kv = __ldg(col + b);
+                const int sb = v.slot_of(b);
+                stream[sb * kCols + sj] = kv;
+                stream[sj * kCols + sb] = make_float4(kv.x, kv.z, kv.y, kv.w); // transposed: Bp, Bm swapped
             }
         }
         __syncthreads();
         }
+        if (cw >= 0) {
+#pragma unroll
+            for (int i = 0; i < TR * C; ++i) {
+                const float4 kv = stream[(cw * TR + i % TR) * kCols + 32 * (i / TR) + lane];
+                tA[i] = kv.x;
+                tP[i] = kv.y;
+                tM[i] = kv.z;
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // these accesses before the columns' copies
+        __syncthreads();
 
         // ---------------- the steps, each warp in its role ----------------
         // Two barriers a step: phase 1 (corrections; the pair that enters joins the tile), phase 2 (the window's
@@ -393,30 +414,33 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
             const float2* cu = cs + cw * TR;
             float2* my_red = reinterpret_cast<float2*>(red + cw * 2 * kCols) + lane;
             auto window_update = [&](float g0, float g1, int jn) {
-                f32x2 x[C], y[C];
+                // (this warp's share of the entering pair's start is summed beside the products: its shuffles wait on
+                // nothing here)
+                const float g = warp_sum_halves(g0, g1, lane);
+                const float s0 = __shfl_sync(0xffffffffu, g, 0), s1 = __shfl_sync(0xffffffffu, g, 16);
+                float x0[C], x1[C], y0[C], y1[C];
 #pragma unroll
-                for (int j = 0; j < C; ++j) x[j] = y[j] = 0ull; // (+0, +0)
+                for (int j = 0; j < C; ++j) x0[j] = x1[j] = y0[j] = y1[j] = 0.f;
 #pragma unroll
                 for (int k = 0; k < TR; ++k) {
                     const float2 c = cu[k];
-                    const f32x2 c0 = pack2(c.x, c.x), c1 = pack2(c.y, c.y);
 #pragma unroll
                     for (int j = 0; j < C; ++j) {
-                        x[j] = fma2(c0, tX[j * TR + k], x[j]);
-                        y[j] = fma2(c1, tY[j * TR + k], y[j]);
+                        x0[j] = fmaf(c.x, tA[j * TR + k], x0[j]);
+                        x1[j] = fmaf(c.x, tP[j * TR + k], x1[j]);
+                        y0[j] = fmaf(c.y, tM[j * TR + k], y0[j]);
+                        y1[j] = fmaf(c.y, tA[j * TR + k], y1[j]);
                     }
                 }
-                // this warp's share of the entering pair's start (beside the products: its shuffles wait on nothing)
-                const float g = warp_sum_halves(g0, g1, lane);
-                const f32x2 start = pack2(__shfl_sync(0xffffffffu, g, 0), __shfl_sync(0xffffffffu, g, 16));
 #pragma unroll
-                for (int j = 0; j < C; ++j) my_red[32 * j] = unpack2(add2(add2(x[j], y[j]), j == jn ? start : 0ull));
+                for (int j = 0; j < C; ++j)
+                    my_red[32 * j] = make_float2(x0[j] + y0[j] + (j == jn ? s0 : 0.f), x1[j] + y1[j] + (j == jn ? s1 : 0.f));
             };
             step_sync<1, kAll>(); // the window's coefficients are in cs
             if (js.used_beforeP > 0) window_update(0.f, 0.f, -1);
             // the pair n entering next: its slot, the place of its column
             int qn, n = js.hi0;
-            const int capP = js.capP, qP = cm.qP, n_first = js.n_first, flo = js.pro ? n_first : 0;
+            const volatile BatchTrainJob& jv = js; // (read in every step: registers are the tile's)
             uint32_t pos = 0;
             {
                 const JobView v(js, cm);
@@ -429,10 +453,11 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                 float g0 = 0.f, g1 = 0.f;
                 const int jn = t + 1 < T0 && lane == (qn & 31) ? qn >> 5 : -1; // the entering pair is in this lane's column jn
                 if (t + 1 < T0) {
-                    // The pair that enters at the next step joins the tile (its corrections are zero until then)
-                    // and its prediction starts, in this warp's share, from the frozen sum and the window's terms
-                    // with the coefficients before this step; the update below adds this step's.
-                    const int lo = max(n + 1 - capP, flo), cnt = max(n_first, n - 1 - qP) - lo;
+                    // The pair that enters at the next step joins the tile (its corrections are zero until then);
+                    // its prediction starts, in this warp's share, from the frozen sum and the window's terms with the
+                    // coefficients before this step; the update below adds this step's
+                    const int n_first = jv.n_first;
+                    const int lo = max(n + 1 - jv.capP, jv.flo), cnt = max(n_first, n - 1 - cm.qP) - lo;
                     const int fi = tid - 32 * kHelpWarps;
                     const bool in = fi < cnt;
                     float4 k1 = stream[(pos + (in ? fi : 0)) & smask];
@@ -442,6 +467,11 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                     a0 = make_float2(lane < TR ? a0.x : 0.f, lane < TR ? a0.y : 0.f);
                     a1 = make_float2(in ? a1.x : 0.f, in ? a1.y : 0.f);
                     if (!in) k1 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (cw == 0) {
+                        const float2 l = lp[((t + 1) & 3) * 32 + lane];
+                        g0 = l.x;
+                        g1 = l.y;
+                    }
                     acc_pair(a0, k0, g0, g1);
                     acc_pair(a1, k1, g0, g1);
 #pragma unroll 1
@@ -449,20 +479,31 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                         acc_pair(ring[(lo + i) & rmask], stream[(pos + i) & smask], g0, g1);
                     const int kn = qn - cw * TR;
                     if (kn >= 0 && kn < TR) { // its row: K(n, j) from column n
-                        f32x2 nx[C], ny[C];
+                        float4 kv[C];
 #pragma unroll
-                        for (int j = 0; j < C; ++j) {
-                            const float4 kv = nbuf[32 * j + lane];
-                            nx[j] = pack2(kv.x, kv.z);
-                            ny[j] = pack2(kv.y, kv.x);
-                        }
+                        for (int j = 0; j < C; ++j) kv[j] = nbuf[32 * j + lane];
 #pragma unroll
-                        for (int i = 0; i < TR * C; ++i) set_if(tX[i], tY[i], nx[i / TR], ny[i / TR], kn, i % TR);
+                        for (int k = 0; k < TR; ++k)
+                            if (kn == k) {
+#pragma unroll
+                                for (int j = 0; j < C; ++j) set(tA[j * TR + k], tP[j * TR + k], tM[j * TR + k], kv[j].x, kv[j].z, kv[j].y);
+                            }
                     }
                     // its column
                     const uint32_t tr = smem_u32(nbuf + cw * TR);
+                    const int mine = lane == (qn & 31), jc = qn >> 5;
+                    if (jc == 0) {
 #pragma unroll
-                    for (int i = 0; i < TR * C; ++i) load_if(tX[i], tY[i], tr + 16 * (i % TR), jn, i / TR);
+                        for (int i = 0; i < TR; ++i) load_if(tA[i], tP[i], tM[i], tr + 16 * i, mine);
+                    } else if (C == 2 || (C > 2 && jc == 1)) {
+                        constexpr int o = C > 1 ? TR : 0;
+#pragma unroll
+                        for (int i = 0; i < TR; ++i) load_if(tA[o + i], tP[o + i], tM[o + i], tr + 16 * i, mine);
+                    } else if (C > 2) {
+                        constexpr int o = C > 2 ? 2 * TR : 0;
+#pragma unroll
+                        for (int i = 0; i < TR; ++i) load_if(tA[o + i], tP[o + i], tM[o + i], tr + 16 * i, mine);
+                    }
                     pos += uint32_t(n + 1 - lo);
                     ++n;
                     qn = qn + 1 == RP ? 0 : qn + 1;
@@ -509,7 +550,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                 cp_commit();
             };
             const bool evicts = v.hiL > capP, ramps = js.ramp != 0;
-            const int flo = v.pro ? n_first : 0;
+            const int flo = js.flo;
             int hi = hi0, s = s0, w = hi0 - s0;
             uint32_t pos = 0; // place of the column of the pair n = hi
             // that column's entries by slot: the window's pairs, the pair that left last, the pair itself
@@ -542,11 +583,9 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                     f32x2 r[RG];
 #pragma unroll
                     for (int g = 0; g < RG; ++g) r[g] = rp[g * kCols];
-                    const float2 sh = *reinterpret_cast<const float2*>(st + (t & 3) * 2);
                     const float4 re = rec[t & 63];
                     if (entered) {
-                        h = sh;
-                        ev = a = make_float2(0.f, 0.f);
+                        h = ev = a = make_float2(0.f, 0.f); // (its whole prediction is in red)
                         y = make_float2(re.x, re.y);
                         rd = re.z;
                     }
@@ -620,9 +659,9 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
             float2 v0 = make_float2(0.f, 0.f), v1 = v0;
             if (has0) v0 = make_float2(vs[lane], vs[N + lane]);
             if (has1) v1 = make_float2(vs[k1], vs[N + k1]);
-            auto sample = [&](int te, int which, int k) {
-                const float* p = xs + (((te - 1) & (2 * kSampleBatch - 1)) * 2 + which) * pitch + k * y_m;
-                return make_float2(p[0], p[y_off]);
+            const float* const x_lane = xs + lane * y_m;
+            auto sample = [&](int at, bool has) { // of the row at `at`, this lane's feature (+ 32 y_m: the second one)
+                return has ? make_float2(x_lane[at], x_lane[at + y_off]) : make_float2(0.f, 0.f);
             };
             const float2 zero = make_float2(0.f, 0.f);
             auto join_v = [&](float2 ab, float2 u0, float2 u1) {
@@ -721,10 +760,13 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                     copy_wait(&xfull[(base_x + seen_x) % kSampleGroups], ((base_x + seen_x) / kSampleGroups) & 1u, abort_flag);
                     ++seen_x;
                 }
-                const float2 x0 = has0 ? sample(te, 0, lane) : zero, x1 = has1 ? sample(te, 0, k1) : zero;
+                const int at = ((te - 1) & (2 * kSampleBatch - 1)) * 2 * pitch;
+                const float2 x0 = sample(at, has0), x1 = sample(at + 32 * y_m, has1);
+                const float2 b0 = sample(at + pitch, has0), b1 = sample(at + pitch + 32 * y_m, has1);
+                const float2 ab = ring[vF & rmask];
                 const float2 ps = prs[te & 63];
                 if (v.frozen_hi(n) > vF) { // the pair vF joins v
-                    join_v(ring[vF & rmask], has0 ? sample(te, 1, lane) : zero, has1 ? sample(te, 1, k1) : zero);
+                    join_v(ab, b0, b1);
                     ++vF;
                 }
                 float g0 = fmaf(v0.x, x0.x, v0.y * x0.y), g1 = fmaf(v0.x, x0.y, -v0.y * x0.x);
@@ -732,8 +774,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                     g0 = fmaf(v1.x, x1.x, fmaf(v1.y, x1.y, g0));
                     g1 = fmaf(v1.x, x1.y, fmaf(-v1.y, x1.x, g1));
                 }
-                const float g = warp_sum_halves(g0, g1, lane);
-                if ((lane & 15) == 0) st[(te & 3) * 2 + (lane >> 4)] = fmaf(wL, g, lane == 0 ? ps.x : ps.y);
+                lp[(te & 3) * 32 + lane] = make_float2(fmaf(wL, g0, lane == 0 ? ps.x : 0.f), fmaf(wL, g1, lane == 0 ? ps.y : 0.f));
             };
             issue(min(lead, T0 + batch)); // (steps before lead)
             if (1 < T0) sample_issue(1);
@@ -828,7 +869,7 @@ template <class S> bool layout_for(int range, int pitch, Layout* l)
     l->pitch = pitch;
     for (l->ring = 256; l->ring < range + 16; l->ring *= 2) {}
     for (int blocks = S::kBlocks; blocks >= 1; --blocks)
-        for (l->stream = 8192; l->stream >= 1024 && l->stream >= 3 * (range + 1); l->stream /= 2)
+        for (l->stream = 8192; l->stream >= S::kMatrix && l->stream >= 3 * (range + 1); l->stream /= 2)
             if (smem_bytes<S>(*l) <= kSmemMax / blocks - 2048) return true;
     return false;
 }
