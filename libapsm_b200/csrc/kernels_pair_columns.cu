@@ -15,6 +15,7 @@
 // Tiles that no column reaches (b > n, or evicted) are skipped: 8192 pilots of
 // 64 antennas write 537 MB instead of 1.07 GB of row-form columns.
 #include "apsm_batch.cuh"
+#include "packed_f32.cuh"
 
 namespace apsm {
 
@@ -23,33 +24,6 @@ namespace {
 constexpr int kTb = 64;  // pairs b per block (16 threads x 4)
 constexpr int kTn = 32;  // columns n per block (16 threads x 2)
 constexpr int kTk = 16;  // antennas per shared-memory chunk
-
-using f32x2 = unsigned long long;
-
-__device__ __forceinline__ f32x2 pack2(float lo, float hi)
-{
-    f32x2 v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
-{
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 
 struct PairColumnsArgs {
     const float* X; // nU x Dp Dedup rows (row 2b = [Re y_b; Im y_b])

@@ -34,6 +34,7 @@
 // frozen entries in chunks of 1024 pairs, the last qP + 2 entries of a column
 // straight into window-slot order.
 #include "apsm_batch.cuh"
+#include "packed_f32.cuh"
 #include "apsm_tc.cuh"
 
 #include <algorithm>
@@ -157,33 +158,6 @@ template <int ID, int THREADS> __device__ __forceinline__ void step_arrive()
 {
     __syncwarp();
     asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
-}
-
-using f32x2 = unsigned long long; // two floats in a register pair, as the packed FP32 instructions take them
-__device__ __forceinline__ f32x2 pack2(float lo, float hi)
-{
-    f32x2 v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
-{
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
 }
 
 // Register updates of the tile in place (selects on the register arrays made the compiler copy the whole tile
