@@ -486,6 +486,7 @@ struct DetectPlan {
     size_t off_rx = 0, off_Y = 0, off_nrm = 0, off_est = 0;
     void* zc_est = nullptr; // host-buffer batch: the caller's estimates as the device writes them in place
     size_t off_aops = 0, off_bops = 0, off_bx = 0, off_lin = 0;
+    int parts = 1;     // CUDA-core detection: blocks that share a sample tile's dictionary chunks
     size_t off_part = 0, off_cnt = 0; // split CUDA-core launches: chunk sums, tile counters
 };
 
@@ -679,21 +680,24 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
         }
 
     const size_t nT = tp.size(), nD = dp.size();
-    // CUDA-core detection: when the batch's sample tiles alone would leave most of the GPU idle
-    // (single requests), the dictionary chunks of each tile are spread over several blocks;
-    // the estimates do not depend on this (launch_batch_detect)
-    int det_parts = 1;
-    {
-        long long tiles_all = 0;
-        int chunks_max = 0;
+    // CUDA-core detection: when a launch's sample tiles alone would leave most of the GPU idle
+    // (single requests, a few detectors of a class), the dictionary chunks of each tile are spread
+    // over several blocks; the estimates do not depend on this (launch_batch_detect).  Eight blocks
+    // of four warps per SM (three at a time): the runs' ends even out, each still does two chunks
+    // or more of a dictionary of 2000 pairs.
+    for (size_t k0 = 0; k0 < nD - nG;) {
+        long long tiles = 0;
+        int chunks = 0;
         const int tile = batch_detect_tile(), chunk = batch_detect_chunk();
-        for (size_t k = 0; k < nD - nG; ++k) {
-            tiles_all += (dp[k].S + tile - 1) / tile;
-            chunks_max = std::max(chunks_max, int((dp[k].Mp + chunk - 1) / chunk));
+        size_t k1 = k0;
+        for (; k1 < nD - nG && dp[k1].cls == dp[k0].cls; ++k1) {
+            tiles += (dp[k1].S + tile - 1) / tile;
+            chunks = std::max(chunks, int((dp[k1].Mp + chunk - 1) / chunk));
         }
-        const long long target = (shape.detect_blocks_per_sm > 0 ? shape.detect_blocks_per_sm : 4LL) * std::max(1, sms);
-        if (tiles_all > 0 && tiles_all < target)
-            det_parts = int(std::min<long long>(std::max(chunks_max, 1), (target + tiles_all - 1) / tiles_all));
+        const long long target = (shape.detect_blocks_per_sm > 0 ? shape.detect_blocks_per_sm : 8LL) * std::max(1, sms);
+        int parts = 1;
+        if (tiles > 0 && tiles < target) parts = int(std::min<long long>(std::max(chunks, 1), (target + tiles - 1) / tiles));
+        for (; k0 < k1; ++k0) dp[k0].parts = parts;
     }
     size_t nCopyIn = 0;
     for (const auto& t : tp) nCopyIn += t.usedP > 0;
@@ -760,12 +764,11 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
     const size_t off_counter = o;
     o = align_up(o + 256, 256);
     const size_t off_dcnt = o;
-    if (det_parts > 1)
-        for (auto& d : dp)
-            if (!d.gram) {
-                d.off_cnt = o;
-                o += sizeof(int) * ((d.S + batch_detect_tile() - 1) / batch_detect_tile());
-            }
+    for (auto& d : dp)
+        if (d.parts > 1) {
+            d.off_cnt = o;
+            o += sizeof(int) * ((d.S + batch_detect_tile() - 1) / batch_detect_tile());
+        }
     o = align_up(o, 256);
     const size_t dcnt_bytes = o - off_dcnt;
     if (host) { // staged host inputs travel with the descriptors
@@ -803,7 +806,7 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
         if (d.gram) {
             d.off_nrm = o; o = align_up(o + sizeof(float) * d.S, 256);
         }
-        if (det_parts > 1 && !d.gram) {
+        if (d.parts > 1) {
             const size_t chunks = (d.Mp + batch_detect_chunk() - 1) / batch_detect_chunk();
             d.off_part = o;
             o = align_up(o + sizeof(float2) * size_t(d.S) * std::max<size_t>(chunks, 1), 256);
@@ -1083,7 +1086,7 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
         auto* ns = q.gram ? reinterpret_cast<float*>(D(q.off_nrm)) : nullptr;
         float2* out = !host ? reinterpret_cast<float2*>(j.est)
                             : zc_est ? static_cast<float2*>(q.zc_est) : reinterpret_cast<float2*>(D(q.off_est));
-        const bool split = det_parts > 1 && !q.gram;
+        const bool split = q.parts > 1;
         h_dj[k] = BatchDetectJob{rx,       d.Y,       d.nrm, d.a,  d.w, out, int(q.S), int(q.Mp), int(d.N), int(d.Np),
                                  d.ew,     split ? reinterpret_cast<float2*>(D(q.off_part)) : nullptr,
                                  split ? reinterpret_cast<int*>(D(q.off_cnt)) : nullptr};
@@ -1350,7 +1353,7 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
                 int tiles = 0;
                 for (size_t k = sg.k0; k < sg.k1; ++k)
                     tiles = std::max(tiles, int((dp[k].S + batch_detect_tile() - 1) / batch_detect_tile()));
-                POOL_CK(launch_batch_detect(d_dj + sg.k0, int(sg.k1 - sg.k0), tiles, det_parts, dp[sg.k0].cls, cfg.wL,
+                POOL_CK(launch_batch_detect(d_dj + sg.k0, int(sg.k1 - sg.k0), tiles, dp[sg.k0].parts, dp[sg.k0].cls, cfg.wL,
                                             cfg.wG, s));
                 L.launches += tiles > 0;
             } else {
