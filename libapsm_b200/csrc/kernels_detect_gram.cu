@@ -12,7 +12,8 @@
 //   gram_bf16x3  compensated: x = xh + xl, d = dh + dl (BF16 each);
 //                x.d ~ xh.dh + xh.dl + xl.dh (3 products, ~2^-16 relative)
 //   gram_tf32    TF32 operands (1 product)
-//   gram_tf32x3  compensated TF32 split (3 products, ~FP32 accuracy)
+//   gram_tf32x3  compensated TF32 split (3 products, ~FP32 accuracy;
+//                kernels_gram_tmem.cu)
 // The squared distance is clamped at 0.  Compensated cross terms (the
 // single-product forms bf16 / tf32): rounding both operands to the format's
 // unit u moves x.d by at most 2u |x||d|, the base-2 exponent
@@ -52,7 +53,7 @@ constexpr int kMaxUsers = 16;
 
 struct GramWorkspace {
     DevBuf<uint8_t> a_ops, b_ops, w_ops; // operand tiles in the UMMA canonical K-major layout
-    DevBuf<float> xn, dn, aw, part, fw, gate;
+    DevBuf<float> xn, dn, aw, part, fw, gate, xd;
     DevBuf<int> err;
     int* h_err = nullptr;
 };
@@ -924,6 +925,68 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
     return APSM_OK;
 }
 
+// TF32 split form: the data tile in tensor memory (kernels_gram_tmem.cu).
+apsm_status run_gram_tmem(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s)
+{
+    constexpr int MODE = kTF32x3;
+    using T = OpTraits<MODE>;
+    GramWorkspace* gw = h->gram;
+    const int ns = int(2 * S);
+    const int M = int(h->used);
+    const int D = int(h->D), Dp = int(h->Dp), U = int(h->U);
+    if (U > kMaxUsers) {
+        h->last_error = "Gram detection supports at most " + std::to_string(kMaxUsers) + " users per detector";
+        return APSM_ERR_UNSUPPORTED;
+    }
+    const int Kp = int(round_up(uint32_t(D), uint32_t(T::kStepK)));
+    const int N = kGramTmemChunk;
+    const int n_tiles = (ns + kTileM - 1) / kTileM;
+    const int n_chunks = std::max(1, (M + N - 1) / N);
+    int splits = std::max(1, std::min(n_chunks, (2 * 148 + n_tiles - 1) / n_tiles));
+    const int cps = (n_chunks + splits - 1) / splits;
+    splits = (n_chunks + cps - 1) / cps;
+
+    cudaError_t e;
+#define GR_CK(x)                                                   \
+    do {                                                           \
+        e = (x);                                                   \
+        if (e != cudaSuccess) return h->cuda_fail(e, #x);          \
+    } while (0)
+    GR_CK(gw->b_ops.ensure(size_t(n_chunks) * N * 2 * Kp * T::kElem));
+    GR_CK(gw->dn.ensure(size_t(n_chunks) * N));
+    GR_CK(gw->xd.ensure(gram_tmem_data_floats(U) * n_chunks));
+    GR_CK(gw->part.ensure(size_t(splits) * U * ns));
+    GR_CK(gw->err.ensure(1));
+    GR_CK(cudaMemsetAsync(gw->err.p, 0, sizeof(int), s));
+
+    const int threads = 256;
+    gram_pack_kernel<MODE><<<std::min(4096, (n_chunks * N * Kp + threads - 1) / threads), threads, 0, s>>>(
+        h->dict_X.p, M, Dp, D, Kp, N, n_chunks, gw->b_ops.p, gw->dn.p);
+    GR_CK(cudaGetLastError());
+
+    GramTmemArgs ga;
+    ga.rows = h->xs.p;
+    ga.b_ops = gw->b_ops.p;
+    ga.xd = gw->xd.p;
+    ga.part = gw->part.p;
+    ga.err = gw->err.p;
+    ga.n_samples = ns;
+    ga.users = U;
+    ga.Kp = Kp;
+    ga.Dp = Dp;
+    ga.chunks_per_split = cps;
+    ga.n_chunks = n_chunks;
+    ga.ewl2 = h->model_params().ew * 1.4426950408889634f;
+    ga.wait_ns = wait_limit_ns();
+    GR_CK(launch_gram_tmem(ga, gw->dn.p, h->dict_a.p, h->cap, M, h->cfg.wG, gw->xd.p, n_tiles, splits, s));
+    gram_finish_kernel<<<(ns + kFinSamples - 1) / kFinSamples, kFinWarps * 32, 0, s>>>(
+        h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns));
+    GR_CK(cudaGetLastError());
+    GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+#undef GR_CK
+    return APSM_OK;
+}
+
 template <int MODE>
 apsm_status run_gram(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s)
 {
@@ -1076,7 +1139,7 @@ apsm_status detect_gram(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t
     case DetectMode::GramBF16: return run_gram<kBF16>(h, S, d_out, s);
     case DetectMode::GramBF16x3: return run_gram<kBF16x3>(h, S, d_out, s);
     case DetectMode::GramTF32: return run_gram<kTF32>(h, S, d_out, s);
-    case DetectMode::GramTF32x3: return run_gram<kTF32x3>(h, S, d_out, s);
+    case DetectMode::GramTF32x3: return run_gram_tmem(h, S, d_out, s);
     default: break;
     }
     h->last_error = "not a Gram detection mode";
