@@ -176,16 +176,21 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
     }
 }
 
-// The same with A in tensor memory (lane = row of A, one 32-bit column per K element for TF32):
-// tmem_a is the column of A's first K element of this step.
+// The same with A in tensor memory (lane = row of A, one 32-bit column per TF32 K element or two
+// BF16 ones): tmem_a is the column of A's first K element of this step.
 template <int MODE>
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate)
 {
-    static_assert(MODE == kTF32 || MODE == kTF32x3, "A from tensor memory: TF32 operands only");
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
-                 "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
+    if constexpr (MODE == kTF32 || MODE == kTF32x3) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
+                     "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
+    } else {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
+                     "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0));
+    }
 }
 
 __device__ __forceinline__ void umma_commit(uint64_t* bar)
@@ -224,6 +229,34 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v)
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 rows x 32 accumulator columns: thread t holds columns 8 g + 2 (t % 4) + {0, 1} of rows t / 4 (v[4 g],
+// v[4 g + 1]) and t / 4 + 8 (v[4 g + 2], v[4 g + 3])
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                   "=r"(r[15])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16], uint32_t (&s)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // (ties the loaded registers to the wait)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]), "+r"(s[i]));
+}
+
+// 16 rows x 16 columns of 32 bits from registers: thread t holds column 4 g + t % 4 of rows t / 4 (v[2 g]) and
+// t / 4 + 8 (v[2 g + 1]) -- as packed BF16 pairs, the columns of tmem_ld_16x32.  Complete after tmem_st_wait.
+__device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 
 // 8 consecutive 32-bit columns of this thread's TMEM lane (complete after tmem_st_wait).

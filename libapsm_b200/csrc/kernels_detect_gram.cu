@@ -36,6 +36,7 @@
 #include "apsm_gram.cuh"
 #include "apsm_kernels.cuh"
 #include "apsm_tc.cuh"
+#include "packed_f32.cuh"
 
 #include <cuda_bf16.h>
 
@@ -486,171 +487,155 @@ __global__ void __launch_bounds__(kFinWarps * 32)
 }
 
 // ------------------------------------------------ two-product form (users >= 4) --
-// The users' contraction on the tensor cores too: per chunk of N dictionary
-// rows, the epilogue turns the Gram tile into kernel values P (128 x N, in the
-// mode's operand format: hi [+ lo]) in shared memory, and a second UMMA
-// (M = 128, N = 16 users, K = N rows) accumulates P W with W the chunk's
-// coefficients a * wG (16 x N, padded with zero users) into tensor memory for
-// the whole dictionary range of the CTA.  The epilogue then costs one
-// exponential and a store per kernel value instead of one FMA per user; the
-// second product rounds P and W to the operand format (split modes: hi/lo, 3
-// products).  Used for the BF16 form with 4 or more users: at N = 64, 16
-// users, a 65536-symbol detection takes 1.66 ms instead of 3.21 ms, the soft
-// outputs moving from 1.4e-6 to 5.2e-5 of the largest output away from the
-// float64 model (decisions unchanged); the TF32 form gains 2 % for a 10x
-// larger error and the split forms lose time (larger P buffers, 3 products),
-// so they keep the one-product kernel.
+// The users' contraction on the tensor cores too (BF16 form): per chunk of 128
+// dictionary rows, the epilogue turns the Gram tile into kernel values P
+// (128 x 128 BF16) in tensor memory, and a second UMMA (M = 128, N = 16 users,
+// K = 128 rows) accumulates P W with W the chunk's coefficients a * wG (16 x 128,
+// padded with zero users) into tensor memory for the whole dictionary range of
+// the CTA.  The epilogue then costs one exponential and half a conversion per
+// kernel value instead of one FMA per user; the second product rounds P and W
+// to BF16.  Used with 4 or more users: the soft outputs move from 1.4e-6 to
+// 5.2e-5 of the largest output away from the float64 model (decisions
+// unchanged, 64 antennas, 16 users); the TF32 form would gain 2 % for a 10x
+// larger error, so the other forms keep the one-product kernel.
+//
+// Bound: the special function unit (131072 x 16384 exponentials: 0.47 ms) and the
+// tensor cores (0.40 ms).  What stood in the way: shared memory (with the data
+// tile and P there, products, stores and the norms' broadcasts came to 1900
+// cycles a chunk against 1024 of exponentials), the issue of the products (their
+// descriptors were built one by one, 100 cycles each) and the chain of one chunk.
+// So the data tile (converted from the packed rows) and P are tensor-memory
+// operands, the epilogue loads two columns by four rows a thread, the
+// dictionary rows have a ring of their own (freed by the Gram tile; coefficients
+// and norms stay until the users' product), even and odd chunks have their own
+// eight epilogue warps, and the users' product follows two Gram tiles behind.
 constexpr int kUsers2 = 16; // UMMA N of the users' product
+constexpr int kN2 = 128;    // dictionary rows per chunk: tensor memory holds two Gram buffers and the users' 16 columns
+constexpr int kStages2 = 4; // chunks' rows in flight
+constexpr int kXStages2 = 4; // chunks' coefficients and norms in flight
+constexpr int kEpiWarps2 = 16;
+constexpr int kGroup2 = kEpiWarps2 / 2; // warps of an even or odd chunk
+constexpr int kThreads2 = (kEpiWarps2 + 2) * 32;
+constexpr int kXd2 = 2 * kN2 + 4; // chunk norms, fix weights, gate
 
 struct Gram2Args {
-    const uint8_t* a_ops; // data tiles (kTileM rows)
-    const uint8_t* b_ops; // dictionary chunks (N rows)
-    const uint8_t* w_ops; // per chunk: W, 16 rows x N (K), canonical K-major, hi [| lo]
-    const float* xn;      // data norms
+    const float* rows;    // data rows (n_samples x Dp, FP32)
+    const uint8_t* b_ops; // dictionary chunks (kN2 rows)
+    const uint8_t* w_ops; // per chunk: W, 16 rows x kN2 (K), canonical K-major
     const float* dn;      // dictionary norms (Mpad)
     const float* fw;      // fix weights (Mpad)
     const float* gate;    // per chunk: max fw, max fw |ewl2 dn|, 0, 0
-    const float* xrows;   // data rows (n_samples x Dp, FP32) for the exact recompute
-    const float* drows;   // dictionary rows (M x Dp, FP32)
+    const float* drows;   // dictionary rows (M x Dp, FP32) for the exact recompute
     float* part;          // splits x users x n_samples partial sums
     int* err;
-    int n_samples, users, Kp, N, Dp, D;
+    int n_samples, users, Kp, Dp, D;
     int chunks_per_split, n_chunks;
-    int stages;
     float ewl2; // ew * log2(e)
     unsigned long long wait_ns; // limit of the bounded waits
 };
 
-// 16 kernel values of one data row (columns col .. col + 15 of the chunk) into the
-// kernel-value operand P (row r; hi [and lo]).  CHECK: entries whose error bound
-// exceeds kFixEps are returned as bits of the mask (their P entries are rewritten).
-template <int MODE, bool CHECK>
-__device__ __forceinline__ uint32_t kernel_values16(const float* gv, const float* sd, int N, int col, float xn,
-                                                    float ewl2, uint8_t* p, int r)
+// Tensor memory columns: two Gram buffers, the users' sums, the data tile and two P buffers (BF16 pairs)
+constexpr uint32_t kTmUsers = 2 * kN2, kTmA = 320, kTmP = 384;
+
+// 32 columns (sd: their norms, fix weights kN2 further) of four rows: thread t's columns 8 e + 2 (t % 4) + {0, 1}
+// of rows t / 4 + 8 m, Gram values v as loaded, kernel values as BF16 pairs into p[m / 2][2 e + m % 2].  CHECK:
+// entries whose error bound exceeds kFixEps are returned as bits 8 m + 2 e + {0, 1} of the mask (p is rewritten).
+template <bool CHECK>
+__device__ __forceinline__ uint32_t kernel_values(const uint32_t (&v)[2][16], const float* sd, const f32x2 (&xn)[4],
+                                                  float ewl2, uint32_t (&p)[2][8])
 {
-    using T = OpTraits<MODE>;
     uint32_t mask = 0u;
+    const f32x2 minus2 = pack2(-2.f, -2.f), ew2 = pack2(ewl2, ewl2);
 #pragma unroll
-    for (int j0 = 0; j0 < 16; j0 += T::kChunk) {
-        // one 16-byte K chunk of this row: hi, and lo for split modes
-        uint32_t hw[4] = {0u, 0u, 0u, 0u}, lw[4] = {0u, 0u, 0u, 0u};
-        float kv[T::kChunk];
+    for (int e = 0; e < 4; ++e) {
+        const f32x2 dn = *reinterpret_cast<const f32x2*>(sd + 8 * e);
+        f32x2 fw = 0ull;
+        if constexpr (CHECK) fw = *reinterpret_cast<const f32x2*>(sd + kN2 + 8 * e);
 #pragma unroll
-        for (int e = 0; e < T::kChunk; ++e) {
-            const int j = j0 + e;
-            const float t = xn + sd[col + j];
-            kv[e] = ex2(ewl2 * fmaxf(fmaf(-2.f, gv[j], t), 0.f));
-            if constexpr (CHECK)
-                if (kv[e] * (ewl2 * t) * sd[N + col + j] < -1.f) mask |= 1u << j;
-        }
-        if constexpr (MODE == kBF16) {
-            // pairs converted by one instruction each (round to nearest)
-#pragma unroll
-            for (int e = 0; e < T::kChunk; e += 2) {
-                const __nv_bfloat162 v2 = __floats2bfloat162_rn(kv[e], kv[e + 1]);
-                hw[e >> 1] = *reinterpret_cast<const uint32_t*>(&v2);
+        for (int m = 0; m < 4; ++m) {
+            const uint32_t* const g = v[m >> 1] + 4 * e + 2 * (m & 1);
+            const f32x2 t = add2(xn[m], dn);
+            const float2 d2 = unpack2(fma2(minus2, pack2(__uint_as_float(g[0]), __uint_as_float(g[1])), t));
+            const float2 x = unpack2(mul2(ew2, pack2(fmaxf(d2.x, 0.f), fmaxf(d2.y, 0.f))));
+            const float k0 = ex2(x.x), k1 = ex2(x.y);
+            if constexpr (CHECK) {
+                const float2 b = unpack2(mul2(pack2(k0, k1), mul2(mul2(ew2, t), fw)));
+                if (b.x < -1.f) mask |= 1u << (8 * m + 2 * e);
+                if (b.y < -1.f) mask |= 2u << (8 * m + 2 * e);
             }
-        } else {
-#pragma unroll
-            for (int e = 0; e < T::kChunk; ++e) {
-                float hi, lo;
-                split_operand<MODE>(kv[e], &hi, &lo);
-                if constexpr (T::kTF) {
-                    hw[e] = __float_as_uint(hi);
-                    lw[e] = __float_as_uint(lo);
-                } else {
-                    hw[e >> 1] |= uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(hi))) << (16 * (e & 1));
-                    lw[e >> 1] |= uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(lo))) << (16 * (e & 1));
-                }
-            }
+            const __nv_bfloat162 k2 = __floats2bfloat162_rn(k0, k1); // (round to nearest)
+            p[m >> 1][2 * e + (m & 1)] = *reinterpret_cast<const uint32_t*>(&k2);
         }
-        const int kc = (col + j0) / T::kChunk;
-        const size_t off = size_t(kc) * (kTileM * 16) + (r >> 3) * 128 + (r & 7) * 16;
-        *reinterpret_cast<uint4*>(p + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-        if constexpr (T::kSplit)
-            *reinterpret_cast<uint4*>(p + size_t(N / T::kChunk) * (kTileM * 16) + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
     }
     return mask;
 }
 
-// W chunks: element (u, k) = a[u][c N + k] * wG (0 past M and for u >= users)
-template <int MODE>
-__global__ void gram_pack_w_kernel(const float* __restrict__ a, size_t a_stride, int users, int M, int N, int n_chunks,
-                                   float wG, uint8_t* __restrict__ w_ops)
+// W chunks: element (u, k) = a[u][c kN2 + k] * wG (0 past M and for u >= users)
+__global__ void gram_pack_w_kernel(const float* __restrict__ a, size_t a_stride, int users, int M, int n_chunks, float wG,
+                                   uint8_t* __restrict__ w_ops)
 {
-    using T = OpTraits<MODE>;
-    const int KE2 = T::kSplit ? 2 * N : N;
-    const size_t total = size_t(n_chunks) * kUsers2 * N;
-    for (size_t idx = blockIdx.x * size_t(blockDim.x) + threadIdx.x; idx < total; idx += size_t(gridDim.x) * blockDim.x) {
-        const int k = int(idx % N);
-        const size_t rest = idx / N;
-        const int u = int(rest % kUsers2), c = int(rest / kUsers2);
-        const int b = c * N + k;
+    const int total = n_chunks * kUsers2 * kN2;
+    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+        const int k = idx % kN2, u = idx / kN2 % kUsers2, c = idx / (kN2 * kUsers2);
+        const int b = c * kN2 + k;
         const float v = (u < users && b < M) ? __fmul_rn(a[size_t(u) * a_stride + b], wG) : 0.f;
-        float hi, lo;
-        split_operand<MODE>(v, &hi, &lo);
-        uint8_t* tile = w_ops + size_t(c) * kUsers2 * KE2 * T::kElem;
-        put_operand<MODE>(tile, kUsers2, u, k, hi);
-        if constexpr (T::kSplit) put_operand<MODE>(tile, kUsers2, u, N + k, lo);
+        put_operand<kBF16>(w_ops + size_t(c) * kUsers2 * kN2 * 2, kUsers2, u, k, v);
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kThreads, 1) gram_detect2_kernel(Gram2Args g)
+__global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
 {
+    constexpr int MODE = kBF16, N = kN2, NS = kStages2, NX = kXStages2;
     using T = OpTraits<MODE>;
     extern __shared__ __align__(1024) uint8_t smem[];
-    const int N = g.N, NS = g.stages;
-    const int KE = T::kSplit ? 2 * g.Kp : g.Kp;
-    const int KE2 = T::kSplit ? 2 * N : N; // K extent of the second product's operands
-    const uint32_t a_bytes = uint32_t(kTileM) * KE * T::kElem;
-    const uint32_t b_bytes = uint32_t(N) * KE * T::kElem;
-    const uint32_t w_bytes = uint32_t(kUsers2) * KE2 * T::kElem;
-    const uint32_t p_bytes = uint32_t(kTileM) * KE2 * T::kElem;
-    uint8_t* sA = smem;
-    uint8_t* sB = sA + a_bytes;                          // [NS] chunk rows
-    uint8_t* sW = sB + size_t(NS) * b_bytes;             // [NS] chunk coefficients
-    uint8_t* sP = sW + size_t(NS) * w_bytes;             // [2] kernel values
-    const int sd_stride = 2 * N + 4;                     // chunk norms, fix weights, gate
-    float* sD = reinterpret_cast<float*>(sP + 2 * size_t(p_bytes)); // [NS][sd_stride]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sD + size_t(NS) * sd_stride);
-    uint64_t* full = bars;             // [NS]
-    uint64_t* empty = bars + NS;       // [NS]
-    uint64_t* tfull = bars + 2 * NS;   // [2]
-    uint64_t* tempty = tfull + 2;      // [2]
-    uint64_t* pfull = tempty + 2;      // [2]
-    uint64_t* pempty = pfull + 2;      // [2]
-    uint64_t* afull = pempty + 2;      // [1]
-    uint64_t* done = afull + 1;        // [1] every product of the CTA completed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const uint32_t b_bytes = uint32_t(N) * g.Kp * T::kElem;
+    constexpr uint32_t w_bytes = kUsers2 * N * T::kElem;
+    uint8_t* const sB = smem;                           // [NS] chunk rows
+    uint8_t* const sW = sB + size_t(NS) * b_bytes;      // [NX] chunk coefficients
+    float* const sD = reinterpret_cast<float*>(sW + size_t(NX) * w_bytes); // [NX][kXd2]
+    float* const sxn = sD + NX * kXd2;                  // [kTileM] data norms
+    uint64_t* const bars = reinterpret_cast<uint64_t*>(sxn + kTileM);
+    uint64_t* const full = bars;             // [NS]
+    uint64_t* const empty = full + NS;       // [NS]
+    uint64_t* const xfull = empty + NS;      // [NX]
+    uint64_t* const xempty = xfull + NX;     // [NX]
+    uint64_t* const tfull = xempty + NX;     // [2]
+    uint64_t* const tempty = tfull + 2;      // [2]
+    uint64_t* const pfull = tempty + 2;      // [2]
+    uint64_t* const pempty = pfull + 2;      // [2]
+    uint64_t* const afull = pempty + 2;      // [1]
+    uint64_t* const done = afull + 1;        // [1] every product of the CTA completed
+    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x, split = blockIdx.y;
     const int c0 = split * g.chunks_per_split;
     const int c1 = min(g.n_chunks, c0 + g.chunks_per_split);
     const int nch = max(0, c1 - c0);
-    uint32_t ncols = 32;
-    while (ncols < uint32_t(2 * N + kUsers2)) ncols <<= 1;
-    const uint32_t acc2 = uint32_t(2 * N); // column of the users' accumulator
+    constexpr uint32_t ncols = 512;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NS; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1 + kEpiWarps);
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < NX; ++s) {
+            mbar_init(&xfull[s], 1);
+            mbar_init(&xempty[s], 1 + kGroup2);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&tfull[s], 1);
-            mbar_init(&tempty[s], kEpiWarps);
-            mbar_init(&pfull[s], kEpiWarps);
+            mbar_init(&tempty[s], kGroup2);
+            mbar_init(&pfull[s], kGroup2);
             mbar_init(&pempty[s], 1);
         }
-        mbar_init(afull, 1);
+        mbar_init(afull, kEpiWarps2);
         mbar_init(done, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kEpiWarps + 1) {
+    if (warp == kEpiWarps2 + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(ncols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -660,82 +645,76 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect2_kernel(Gram2Args g)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == kEpiWarps) {
-        // ---------------- producer: data tile once, then dictionary chunks with their W and norms ----------------
+    if (warp == kEpiWarps2) {
+        // ---------------- producer: dictionary chunks with their W and norms ----------------
         if (lane == 0) {
-            mbar_expect_tx(afull, a_bytes);
-            bulk_g2s(sA, g.a_ops + size_t(tile) * a_bytes, a_bytes, afull);
-            int issued = 0;
+            int issued = 0, xissued = 0;
             for (int i = 0; i < nch; ++i) {
-                const int s = i % NS;
+                const int s = i % NS, x = i % NX, c = c0 + i;
                 if (i >= NS && !mbar_wait(&empty[s], ((i / NS) - 1) & 1, abort_flag, g.wait_ns)) break;
                 ++issued;
-                const int c = c0 + i;
-                mbar_expect_tx(&full[s], b_bytes + w_bytes + uint32_t(sd_stride) * 4);
+                mbar_expect_tx(&full[s], b_bytes);
                 bulk_g2s(sB + size_t(s) * b_bytes, g.b_ops + size_t(c) * b_bytes, b_bytes, &full[s]);
-                bulk_g2s(sW + size_t(s) * w_bytes, g.w_ops + size_t(c) * w_bytes, w_bytes, &full[s]);
-                float* sd = sD + size_t(s) * sd_stride;
-                bulk_g2s(sd, g.dn + size_t(c) * N, uint32_t(N) * 4, &full[s]);
-                bulk_g2s(sd + N, g.fw + size_t(c) * N, uint32_t(N) * 4, &full[s]);
-                bulk_g2s(sd + 2 * N, g.gate + size_t(c) * 4, 16, &full[s]);
+                if (i >= NX && !mbar_wait(&xempty[x], ((i / NX) - 1) & 1, abort_flag, g.wait_ns)) break;
+                ++xissued;
+                mbar_expect_tx(&xfull[x], w_bytes + kXd2 * 4);
+                bulk_g2s(sW + size_t(x) * w_bytes, g.w_ops + size_t(c) * w_bytes, w_bytes, &xfull[x]);
+                float* sd = sD + size_t(x) * kXd2;
+                bulk_g2s(sd, g.dn + size_t(c) * N, uint32_t(N) * 4, &xfull[x]);
+                bulk_g2s(sd + N, g.fw + size_t(c) * N, uint32_t(N) * 4, &xfull[x]);
+                bulk_g2s(sd + 2 * N, g.gate + size_t(c) * 4, 16, &xfull[x]);
             }
-            mbar_drain(afull, 0);
             for (int i = max(0, issued - NS); i < issued; ++i) mbar_drain(&full[i % NS], (i / NS) & 1);
+            for (int i = max(0, xissued - NX); i < xissued; ++i) mbar_drain(&xfull[i % NX], (i / NX) & 1);
         }
-    } else if (warp == kEpiWarps + 1) {
-        // ---------------- MMA issuer: Gram tile of chunk i, then the users' product of chunk i - 1 ----------------
+    } else if (warp == kEpiWarps2 + 1) {
+        // ---------------- MMA issuer: Gram tile of chunk i, then the users' product of chunk i - 2 ----------------
         if (lane == 0 && mbar_wait(afull, 0, abort_flag, g.wait_ns)) {
             const uint32_t idesc = instr_desc<MODE>(kTileM, N);
             const uint32_t idesc2 = instr_desc<MODE>(kTileM, kUsers2);
-            const uint32_t lbo_a = kTileM * 16, lbo_b = uint32_t(N) * 16, lbo_w = kUsers2 * 16;
-            const int ksteps = g.Kp / T::kStepK, ksteps2 = N / T::kStepK;
-            const int lo_off = g.Kp / T::kChunk, lo_off2 = N / T::kChunk;
+            constexpr uint32_t lbo = kTileM * 16, lbo_w = kUsers2 * 16;
+            const int ksteps = g.Kp / T::kStepK;
+            constexpr int ksteps2 = N / T::kStepK;
+            // One thread issues everything: descriptors are built once, a K step or a buffer is an addition to
+            // their address field (units of 16 bytes).  Building them for every product took 100 cycles each,
+            // more than the products.
+            constexpr uint64_t kStep = 2 * lbo / 16, kStepW = 2 * lbo_w / 16;
+            const uint64_t db = smem_desc(sB, lbo, 128), dw = smem_desc(sW, lbo_w, 128);
+            constexpr uint32_t kStepA = T::kStepK / 2; // tensor-memory columns of a K step
             bool ok = true;
             auto product2 = [&](int j) {
-                const int pb = j & 1, sj = j % NS;
-                if (!mbar_wait(&pfull[pb], (j >> 1) & 1, abort_flag, g.wait_ns)) {
+                const int pb = j & 1, xj = j % NX;
+                if (!mbar_wait(&xfull[xj], (j / NX) & 1, abort_flag, g.wait_ns) ||
+                    !mbar_wait(&pfull[pb], (j >> 1) & 1, abort_flag, g.wait_ns)) {
                     ok = false;
                     return;
                 }
                 tc_fence_after();
-                const uint8_t* p = sP + size_t(pb) * p_bytes;
-                const uint8_t* w = sW + size_t(sj) * w_bytes;
-                for (int kk = 0; kk < ksteps2; ++kk) {
-                    const uint64_t ah = smem_desc(p + size_t(2 * kk) * lbo_a, lbo_a, 128);
-                    const uint64_t bh = smem_desc(w + size_t(2 * kk) * lbo_w, lbo_w, 128);
-                    umma<MODE>(tmem + acc2, ah, bh, idesc2, (j > 0 || kk > 0) ? 1u : 0u);
-                    if constexpr (T::kSplit) {
-                        const uint64_t al = smem_desc(p + size_t(lo_off2 + 2 * kk) * lbo_a, lbo_a, 128);
-                        const uint64_t bl = smem_desc(w + size_t(lo_off2 + 2 * kk) * lbo_w, lbo_w, 128);
-                        umma<MODE>(tmem + acc2, ah, bl, idesc2, 1u);
-                        umma<MODE>(tmem + acc2, al, bh, idesc2, 1u);
-                    }
-                }
+                const uint64_t w = dw + uint64_t(xj) * (w_bytes / 16);
+                const uint32_t p = tmem + kTmP + uint32_t(pb * (N / 2));
+                umma_ts<MODE>(tmem + kTmUsers, p, w, idesc2, j > 0 ? 1u : 0u);
+#pragma unroll
+                for (int kk = 1; kk < ksteps2; ++kk)
+                    umma_ts<MODE>(tmem + kTmUsers, p + kk * kStepA, w + kk * kStepW, idesc2, 1u);
                 umma_commit(&pempty[pb]); // kernel-value buffer free once these products completed
-                umma_commit(&empty[sj]);  // the chunk's rows and coefficients too
+                umma_commit(&xempty[xj]); // the chunk's coefficients too
             };
             for (int i = 0; i < nch && ok; ++i) {
                 const int s = i % NS, buf = i & 1;
                 if (!mbar_wait(&full[s], (i / NS) & 1, abort_flag, g.wait_ns)) break;
                 if (i >= 2 && !mbar_wait(&tempty[buf], ((i >> 1) - 1) & 1, abort_flag, g.wait_ns)) break;
                 tc_fence_after();
-                const uint8_t* b = sB + size_t(s) * b_bytes;
+                const uint64_t b = db + uint64_t(s) * (b_bytes / 16);
                 const uint32_t d = tmem + uint32_t(buf * N);
-                for (int kk = 0; kk < ksteps; ++kk) {
-                    const uint64_t ah = smem_desc(sA + size_t(2 * kk) * lbo_a, lbo_a, 128);
-                    const uint64_t bh = smem_desc(b + size_t(2 * kk) * lbo_b, lbo_b, 128);
-                    umma<MODE>(d, ah, bh, idesc, kk > 0 ? 1u : 0u);
-                    if constexpr (T::kSplit) {
-                        const uint64_t al = smem_desc(sA + size_t(lo_off + 2 * kk) * lbo_a, lbo_a, 128);
-                        const uint64_t bl = smem_desc(b + size_t(lo_off + 2 * kk) * lbo_b, lbo_b, 128);
-                        umma<MODE>(d, ah, bl, idesc, 1);
-                        umma<MODE>(d, al, bh, idesc, 1);
-                    }
-                }
+                umma_ts<MODE>(d, tmem + kTmA, b, idesc, 0u);
+#pragma unroll
+                for (int kk = 1; kk < kMaxFeatures / T::kStepK; ++kk)
+                    if (kk < ksteps) umma_ts<MODE>(d, tmem + kTmA + kk * kStepA, b + kk * kStep, idesc, 1u);
                 umma_commit(&tfull[buf]); // Gram tile ready for the epilogue
-                if (i >= 1) product2(i - 1);
+                umma_commit(&empty[s]);   // the chunk's rows are free
+                if (i >= 2) product2(i - 2);
             }
-            if (ok && nch > 0 && !*abort_flag) product2(nch - 1);
+            for (int j = max(0, nch - 2); j < nch && ok && !*abort_flag; ++j) product2(j);
         }
         if (lane == 0) {
             umma_commit(done);
@@ -743,59 +722,112 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect2_kernel(Gram2Args g)
         }
     } else {
         // ---------------- epilogue: kernel values of each chunk into P; at the end the users' sums ----------------
-        const int q = warp & 3, h = warp >> 2;
-        const int r = q * 32 + lane; // row of the tile (tensor-memory lane)
-        const int row = tile * kTileM + r;
-        const bool valid = row < g.n_samples;
-        const float xn = valid ? g.xn[row] : 0.f;
-        constexpr bool kFix = fix_scale<MODE>() > 0.f && !T::kSplit;
-        const float exn_max = kFix ? warp_exn_max(g.ewl2, xn) : 0.f;
-        const int half = N / 2;
-        bool ok = true;
-        for (int i = 0; i < nch; ++i) {
-            const int s = i % NS, buf = i & 1, pb = i & 1;
-            if (!mbar_wait(&full[s], (i / NS) & 1, abort_flag, g.wait_ns) ||
-                !mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, g.wait_ns) ||
-                (i >= 2 && !mbar_wait(&pempty[pb], ((i >> 1) - 1) & 1, abort_flag, g.wait_ns))) {
-                ok = false;
-                break;
-            }
-            tc_fence_after();
-            const float* sd = sD + size_t(s) * sd_stride;
-            uint8_t* p = sP + size_t(pb) * p_bytes;
-            const uint32_t trow = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * N);
-            // can any entry of this chunk exceed the bound for a row of this warp?  (warp-uniform)
-            const bool check = kFix && fmaf(exn_max, sd[2 * N], sd[2 * N + 1]) > 1.f;
-            for (int cb = 0; cb < half; cb += 16) {
-                const int col = h * half + cb;
-                float gv[16];
-                tmem_ld16(trow + uint32_t(col), gv);
-                if (!check) {
-                    kernel_values16<MODE, false>(gv, sd, N, col, xn, g.ewl2, p, r);
-                    continue;
+        const int q = warp & 3, group = warp >> 3, half = (warp >> 2 & 1) * (N / 2); // this warp's columns of its chunks
+        const uint32_t tlane = tmem + (uint32_t(q * 32) << 16);
+        const int row = tile * kTileM + q * 32 + lane; // of this thread's tensor-memory lane
+        {
+            // the data tile: K steps warp / 4, + 4, ... of this row; the first warps also the norms
+            const float* const xr = g.rows + size_t(row) * g.Dp;
+            auto load4 = [&](int k) {
+                return row < g.n_samples && k < g.Dp ? __ldg(reinterpret_cast<const float4*>(xr + k))
+                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+            };
+#pragma unroll 2
+            for (int k = 16 * (warp >> 2); k < g.Kp; k += 64) {
+                uint32_t w[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 v = load4(k + 4 * j);
+                    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                    w[2 * j] = *reinterpret_cast<const uint32_t*>(&lo);
+                    w[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&hi);
                 }
-                uint32_t mask = kernel_values16<MODE, true>(gv, sd, N, col, xn, g.ewl2, p, r);
-                if (!valid) mask = 0u;
-                // flagged entries: exact squared distance from the FP32 rows, the value rewritten in P
-                while (mask) {
-                    const int j = __ffs(mask) - 1;
-                    mask &= mask - 1u;
-                    const float d2 = row_distance(g.xrows + size_t(row) * g.Dp,
-                                                  g.drows + size_t((c0 + i) * N + col + j) * g.Dp, g.D);
-                    put_operand<MODE>(p, kTileM, r, col + j, ex2(g.ewl2 * d2));
-                }
+                tmem_st8(tlane + kTmA + uint32_t(k / 2), w);
             }
+            if (warp < 4) {
+                float acc = 0.f;
+#pragma unroll 8
+                for (int k = 0; k < g.Dp; k += 4) {
+                    const float4 v = load4(k);
+                    acc = fmaf(v.x, v.x, acc);
+                    acc = fmaf(v.y, v.y, acc);
+                    acc = fmaf(v.z, v.z, acc);
+                    acc = fmaf(v.w, v.w, acc);
+                }
+                sxn[q * 32 + lane] = acc;
+            }
+            tmem_st_wait();
             tc_fence_before();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // P visible to the tensor cores
+            __syncwarp();
+            if (lane == 0) mbar_arrive(afull);
+            asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps2 * 32) : "memory");
+        }
+        const int r0 = q * 32 + (lane >> 2), cp = 2 * (lane & 3); // rows r0 + 8 m, columns cp, cp + 1 of each eight
+        f32x2 xn[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) xn[m] = pack2(sxn[r0 + 8 * m], sxn[r0 + 8 * m]);
+        const float exn_max = warp_exn_max(g.ewl2, sxn[q * 32 + lane]);
+        bool ok = true;
+        for (int i = group; i < nch; i += 2) { // buffers of the chunk: Gram tile and P number `group`
+            const int x = i % NX, ph = (i >> 1) & 1;
+            ok = mbar_wait(&xfull[x], (i / NX) & 1, abort_flag, g.wait_ns) &&
+                 mbar_wait(&tfull[group], ph, abort_flag, g.wait_ns) &&
+                 (i < 2 || mbar_wait(&pempty[group], ph ^ 1, abort_flag, g.wait_ns));
+            ok = __all_sync(0xffffffffu, ok); // (the loads below are warp-wide)
+            if (!ok) break;
+            tc_fence_after();
+            const float* sd = sD + size_t(x) * kXd2;
+            // can any entry of this chunk exceed the bound for a row of this warp?  (warp-uniform)
+            const bool check = fmaf(exn_max, sd[2 * N], sd[2 * N + 1]) > 1.f;
+#pragma unroll 1
+            for (int col = half; col < half + N / 2; col += 32) {
+                uint32_t v[2][16], p[2][8];
+                tmem_ld_16x32(tlane + uint32_t(group * N + col), v[0]);
+                tmem_ld_16x32(tlane + (16u << 16) + uint32_t(group * N + col), v[1]);
+                tmem_ld_wait(v[0], v[1]);
+                if (col != half) { // the accumulators are in registers
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[group]);
+                }
+                if (!check) {
+                    kernel_values<false>(v, sd + col + cp, xn, g.ewl2, p);
+                } else {
+                    uint32_t mask = kernel_values<true>(v, sd + col + cp, xn, g.ewl2, p);
+                    // flagged entries: exact squared distance from the FP32 rows, the value replaced
+                    while (mask) {
+                        const int j = __ffs(mask) - 1, fr = tile * kTileM + r0 + 8 * (j >> 3);
+                        mask &= mask - 1u;
+                        if (fr >= g.n_samples) continue;
+                        const float d2 = row_distance(
+                            g.rows + size_t(fr) * g.Dp,
+                            g.drows + size_t((c0 + i) * N + col + cp + 8 * (j >> 1 & 3) + (j & 1)) * g.Dp, g.D);
+                        const uint32_t k = __bfloat16_as_ushort(__float2bfloat16_rn(ex2(g.ewl2 * d2)));
+#pragma unroll
+                        for (int m = 0; m < 4; ++m)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if ((j >> 1) == 4 * m + e) {
+                                    uint32_t& t = p[m >> 1][2 * e + (m & 1)];
+                                    t = (j & 1) ? (t & 0xffffu) | k << 16 : (t & 0xffff0000u) | k;
+                                }
+                    }
+                }
+                const uint32_t tp = tlane + kTmP + uint32_t(group * (N / 2) + col / 2);
+                __syncwarp();
+                tmem_st_16x16(tp, p[0]);
+                tmem_st_16x16(tp + (16u << 16), p[1]);
+            }
+            tmem_st_wait();
+            tc_fence_before(); // P visible to the tensor cores
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&tempty[buf]);
-                mbar_arrive(&empty[s]);
-                mbar_arrive(&pfull[pb]);
+                mbar_arrive(&xempty[x]);
+                mbar_arrive(&pfull[group]);
             }
         }
-        if (h == 0) {
-            // warps 0-3 read the users' sums of their 32 lanes (tcgen05.ld is warp-wide: the
+        if (warp < 4) {
+            // the first four warps read the users' sums of their 32 lanes (tcgen05.ld is warp-wide: the
             // whole warp loads, the lanes of rows past the end discard)
             float acc[kUsers2];
 #pragma unroll
@@ -803,28 +835,28 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect2_kernel(Gram2Args g)
             const bool have = ok && nch > 0 && mbar_wait(done, 0, abort_flag, g.wait_ns);
             if (__all_sync(0xffffffffu, have)) {
                 tc_fence_after();
-                tmem_ld16(tmem + (uint32_t(q * 32) << 16) + acc2, acc);
+                tmem_ld16(tlane + kTmUsers, acc);
             }
             if (row < g.n_samples)
-                for (int u = 0; u < g.users; ++u) g.part[(size_t(split) * g.users + u) * g.n_samples + row] = acc[u];
+#pragma unroll
+                for (int u = 0; u < kUsers2; ++u)
+                    if (u < g.users) g.part[(size_t(split) * g.users + u) * g.n_samples + row] = acc[u];
         }
     }
 
     tc_fence_before();
     __syncthreads();
-    if (warp == kEpiWarps + 1) {
+    if (warp == kEpiWarps2 + 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
     }
     if (threadIdx.x == 0 && *abort_flag) atomicExch(g.err, 1);
 }
 
-template <int MODE> size_t gram2_smem(int Kp, int N, int stages)
+size_t gram2_smem(int Kp)
 {
-    using T = OpTraits<MODE>;
-    const size_t KE = T::kSplit ? 2 * Kp : Kp, KE2 = T::kSplit ? 2 * N : N;
-    return size_t(kTileM) * KE * T::kElem + size_t(stages) * (size_t(N) * KE * T::kElem + kUsers2 * KE2 * T::kElem) +
-           2 * size_t(kTileM) * KE2 * T::kElem + size_t(stages) * (2 * N + 4) * 4 + (2 * stages + 10) * 8 + 16;
+    return size_t(kStages2) * kN2 * Kp * 2 + size_t(kXStages2) * kUsers2 * kN2 * 2 +
+           sizeof(float) * (kXStages2 * kXd2 + kTileM) + (2 * kStages2 + 2 * kXStages2 + 10) * 8 + 16;
 }
 
 template <int MODE, int NU> void launch_gram(const GramArgs& ga, int n_tiles, int splits, size_t smem, cudaStream_t s,
@@ -836,19 +868,13 @@ template <int MODE, int NU> void launch_gram(const GramArgs& ga, int n_tiles, in
     *e = cudaGetLastError();
 }
 
-template <int MODE>
-apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s, int Kp, int N, int stages)
+apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s, int Kp)
 {
-    using T = OpTraits<MODE>;
-    if (2 * N + kUsers2 > 512) { // the kernel's tensor memory: 2 N + 16 columns rounded up to a power of two
-        h->last_error = "two-product Gram detection: chunk of " + std::to_string(N) + " rows exceeds tensor memory";
-        return APSM_ERR_UNSUPPORTED;
-    }
+    constexpr int MODE = kBF16, N = kN2;
     GramWorkspace* gw = h->gram;
     const int ns = int(2 * S);
     const int M = int(h->used);
     const int D = int(h->D), Dp = int(h->Dp), U = int(h->U);
-    const int KE = T::kSplit ? 2 * Kp : Kp, KE2 = T::kSplit ? 2 * N : N;
     const int n_tiles = (ns + kTileM - 1) / kTileM;
     const int n_chunks = std::max(1, (M + N - 1) / N);
     const int Mpad = n_chunks * N;
@@ -862,10 +888,8 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
         e = (x);                                                   \
         if (e != cudaSuccess) return h->cuda_fail(e, #x);          \
     } while (0)
-    GR_CK(gw->a_ops.ensure(size_t(n_tiles) * kTileM * KE * T::kElem));
-    GR_CK(gw->b_ops.ensure(size_t(n_chunks) * N * KE * T::kElem));
-    GR_CK(gw->w_ops.ensure(size_t(n_chunks) * kUsers2 * KE2 * T::kElem));
-    GR_CK(gw->xn.ensure(size_t(n_tiles) * kTileM));
+    GR_CK(gw->b_ops.ensure(size_t(n_chunks) * N * Kp * 2));
+    GR_CK(gw->w_ops.ensure(size_t(n_chunks) * kUsers2 * N * 2));
     GR_CK(gw->dn.ensure(Mpad));
     GR_CK(gw->fw.ensure(Mpad));
     GR_CK(gw->gate.ensure(size_t(4) * n_chunks));
@@ -876,46 +900,39 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
     const float ewl2 = h->model_params().ew * 1.4426950408889634f;
 
     const int threads = 256;
-    gram_pack_kernel<MODE><<<std::min(4096, (n_tiles * kTileM * Kp + threads - 1) / threads), threads, 0, s>>>(
-        h->xs.p, ns, Dp, D, Kp, kTileM, n_tiles, gw->a_ops.p, gw->xn.p);
-    GR_CK(cudaGetLastError());
     gram_pack_kernel<MODE><<<std::min(4096, (n_chunks * N * Kp + threads - 1) / threads), threads, 0, s>>>(
         h->dict_X.p, M, Dp, D, Kp, N, n_chunks, gw->b_ops.p, gw->dn.p);
     GR_CK(cudaGetLastError());
     gram_fix_kernel<MODE><<<n_chunks, 256, 0, s>>>(h->dict_a.p, h->cap, U, M, N, h->cfg.wG, ewl2, gw->dn.p, gw->fw.p,
                                                    gw->gate.p);
     GR_CK(cudaGetLastError());
-    gram_pack_w_kernel<MODE><<<std::min(4096, (n_chunks * kUsers2 * N + threads - 1) / threads), threads, 0, s>>>(
-        h->dict_a.p, h->cap, U, M, N, n_chunks, h->cfg.wG, gw->w_ops.p);
+    gram_pack_w_kernel<<<std::min(4096, (n_chunks * kUsers2 * N + threads - 1) / threads), threads, 0, s>>>(
+        h->dict_a.p, h->cap, U, M, n_chunks, h->cfg.wG, gw->w_ops.p);
     GR_CK(cudaGetLastError());
 
     Gram2Args ga;
-    ga.a_ops = gw->a_ops.p;
+    ga.rows = h->xs.p;
     ga.b_ops = gw->b_ops.p;
     ga.w_ops = gw->w_ops.p;
-    ga.xn = gw->xn.p;
     ga.dn = gw->dn.p;
     ga.fw = gw->fw.p;
     ga.gate = gw->gate.p;
-    ga.xrows = h->xs.p;
     ga.drows = h->dict_X.p;
     ga.part = gw->part.p;
     ga.err = gw->err.p;
     ga.n_samples = ns;
     ga.users = U;
     ga.Kp = Kp;
-    ga.N = N;
     ga.Dp = Dp;
     ga.D = D;
     ga.chunks_per_split = cps;
     ga.n_chunks = n_chunks;
-    ga.stages = stages;
     ga.ewl2 = ewl2;
     ga.wait_ns = wait_limit_ns();
-    // >= 120 KB keeps one CTA per SM: its tensor memory (up to 512 columns) is never contended
-    const size_t smem = std::max<size_t>(gram2_smem<MODE>(Kp, N, stages) + 1024, 120 * 1024);
-    GR_CK(cudaFuncSetAttribute(gram_detect2_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    gram_detect2_kernel<MODE><<<dim3(n_tiles, splits), kThreads, smem, s>>>(ga);
+    // >= 120 KB keeps one CTA per SM: its tensor memory (512 columns) is never contended
+    const size_t smem = std::max<size_t>(gram2_smem(Kp) + 1024, 120 * 1024);
+    GR_CK(cudaFuncSetAttribute(gram_detect2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    gram_detect2_kernel<<<dim3(n_tiles, splits), kThreads2, smem, s>>>(ga);
     GR_CK(cudaGetLastError());
     gram_finish_kernel<<<(ns + kFinSamples - 1) / kFinSamples, kFinWarps * 32, 0, s>>>(
         h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns));
@@ -1001,16 +1018,11 @@ apsm_status run_gram(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s)
     }
     const int Kp = int(round_up(uint32_t(D), uint32_t(T::kStepK)));
     const int KE = T::kSplit ? 2 * Kp : Kp;
-    if (MODE == kBF16 && U >= 4 && !h->gram_one_product) {
-        // the users' contraction on the tensor cores where its operands fit shared memory; only
-        // in the BF16 form, whose kernel values and coefficients may be BF16 too (in the other
-        // forms the second product's rounding would cost more accuracy than its time saves)
-        // tensor memory: two Gram buffers of n2 columns and the users' 16, rounded up to a power of
-        // two, within the 512 columns of an SM: n2 <= 128
-        for (int n2 = 128; n2 >= 32; n2 /= 2)
-            for (int st2 = kMaxStages; st2 >= 2; --st2)
-                if (gram2_smem<MODE>(Kp, n2, st2) + 1024 <= 220 * 1024) return run_gram2<MODE>(h, S, d_out, s, Kp, n2, st2);
-    }
+    // the users' contraction on the tensor cores; only in the BF16 form, whose kernel values and
+    // coefficients may be BF16 too (in the other forms the second product's rounding would cost
+    // more accuracy than its time saves)
+    if constexpr (MODE == kBF16)
+        if (U >= 4 && !h->gram_one_product) return run_gram2(h, S, d_out, s, Kp);
     // dictionary chunk width and stages: the data tile and the chunk ring within shared memory
     // (chunks of 256 down to 64 columns in 3 stages, then 32 columns in 3 or 2 stages)
     int N = 256, stages = kMaxStages;

@@ -73,25 +73,6 @@ __global__ void chunk_data_kernel(const float* __restrict__ dn, const float* __r
     }
 }
 
-// 16 rows x 32 accumulator columns: thread t holds columns 8 g + 2 (t % 4) + {0, 1} of rows t / 4 (v[4 g],
-// v[4 g + 1]) and t / 4 + 8 (v[4 g + 2], v[4 g + 3])
-__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                   "=r"(r[15])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16], uint32_t (&s)[16])
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    // (ties the loaded registers to the wait)
-#pragma unroll
-    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]), "+r"(s[i]));
-}
-
 template <int NU>
 __global__ void __launch_bounds__(kThreads, 1) gram_tmem_kernel(GramTmemArgs g)
 {
@@ -190,6 +171,11 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tmem_kernel(GramTmemArgs g)
             tc_fence_after();
             const uint32_t idesc = instr_desc<MODE>(kTileM, kN);
             constexpr uint32_t lbo = kN * 16;
+            // One thread issues everything: descriptors are built once, a K step, the lo half or a stage is an
+            // addition to their address field (units of 16 bytes).  Building them for every product took 100
+            // cycles each, about what a product takes.
+            constexpr uint64_t kStep = 2 * lbo / 16;
+            const uint64_t db = smem_desc(sB, lbo, 128), lo_half = half_bytes / 16;
             int n = 0;
             bool ok = true;
             for (int i = 0; i < nch && ok; ++i) {
@@ -203,16 +189,16 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tmem_kernel(GramTmemArgs g)
                         break;
                     }
                     tc_fence_after();
-                    const uint8_t* const b = sB + size_t(s) * 2 * half_bytes;
+                    const uint64_t bh = db + uint64_t(s) * (2 * lo_half), bl = bh + lo_half;
+                    const uint32_t ah = tmem + kAcol + uint32_t(f * kSliceK), al = ah + uint32_t(Kp);
                     const int steps = min(kSliceK, Kp - f * kSliceK) / T::kStepK;
-                    for (int kk = 0; kk < steps; ++kk) {
-                        // data hi / lo of this K step: T::kStepK tensor-memory columns each
-                        const uint32_t ah = tmem + kAcol + uint32_t(f * kSliceK + kk * T::kStepK);
-                        const uint64_t bh = smem_desc(b + size_t(2 * kk) * lbo, lbo, 128);
-                        const uint64_t bl = smem_desc(b + half_bytes + size_t(2 * kk) * lbo, lbo, 128);
-                        umma_ts<MODE>(d, ah, bh, idesc, (f > 0 || kk > 0) ? 1u : 0u);
-                        umma_ts<MODE>(d, ah, bl, idesc, 1u);
-                        umma_ts<MODE>(d, ah + uint32_t(Kp), bh, idesc, 1u);
+#pragma unroll
+                    for (int kk = 0; kk < kSliceK / T::kStepK; ++kk) {
+                        if (kk >= steps) break;
+                        // data hi / lo of a K step: T::kStepK tensor-memory columns each
+                        umma_ts<MODE>(d, ah + kk * T::kStepK, bh + kk * kStep, idesc, (f > 0 || kk > 0) ? 1u : 0u);
+                        umma_ts<MODE>(d, ah + kk * T::kStepK, bl + kk * kStep, idesc, 1u);
+                        umma_ts<MODE>(d, al + kk * T::kStepK, bh + kk * kStep, idesc, 1u);
                     }
                     umma_commit(&empty[s]);
                 }
