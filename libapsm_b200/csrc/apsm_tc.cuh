@@ -250,15 +250,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16], uint32_t (&s)[16
     for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]), "+r"(s[i]));
 }
 
-// 16 rows x 16 columns of 32 bits from registers: thread t holds column 4 g + t % 4 of rows t / 4 (v[2 g]) and
-// t / 4 + 8 (v[2 g + 1]) -- as packed BF16 pairs, the columns of tmem_ld_16x32.  Complete after tmem_st_wait.
-__device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t (&r)[8])
-{
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-
 // 8 consecutive 32-bit columns of this thread's TMEM lane (complete after tmem_st_wait).
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v)
 {

@@ -487,30 +487,28 @@ __global__ void __launch_bounds__(kFinWarps * 32)
 }
 
 // ------------------------------------------------ two-product form (users >= 4) --
-// The users' contraction on the tensor cores too (BF16 form): per chunk of 128
-// dictionary rows, the epilogue turns the Gram tile into kernel values P
-// (128 x 128 BF16) in tensor memory, and a second UMMA (M = 128, N = 16 users,
-// K = 128 rows) accumulates P W with W the chunk's coefficients a * wG (16 x 128,
-// padded with zero users) into tensor memory for the whole dictionary range of
-// the CTA.  The epilogue then costs one exponential and half a conversion per
-// kernel value instead of one FMA per user; the second product rounds P and W
-// to BF16.  Used with 4 or more users: the soft outputs move from 1.4e-6 to
-// 5.2e-5 of the largest output away from the float64 model (decisions
-// unchanged, 64 antennas, 16 users); the TF32 form would gain 2 % for a 10x
-// larger error, so the other forms keep the one-product kernel.
+// The users' contraction on the tensor cores too (BF16 form): the Gram tile of a
+// chunk of 128 dictionary rows becomes kernel values, and these as BF16 times the
+// chunk's coefficients a * wG (BF16, padded with zero users to 16) add to the
+// users' sums.  The epilogue then costs one exponential and half a conversion
+// per kernel value instead of one FMA per user; the second product rounds kernel
+// values and coefficients to BF16.  Used with 4 or more users: the soft outputs
+// move from 1.4e-6 to 5.2e-5 of the largest output away from the float64 model
+// (decisions unchanged, 64 antennas, 16 users); the TF32 form would gain 2 % for
+// a 10x larger error, so the other forms keep the one-product kernel.
 //
 // Bound: the special function unit (131072 x 16384 exponentials: 0.47 ms) and the
-// tensor cores (0.40 ms).  What stood in the way: shared memory (with the data
-// tile and P there, products, stores and the norms' broadcasts came to 1900
-// cycles a chunk against 1024 of exponentials), the issue of the products (their
-// descriptors were built one by one, 100 cycles each) and the chain of one chunk.
-// So the data tile (converted from the packed rows) and P are tensor-memory
-// operands, the epilogue loads two columns by four rows a thread, the
-// dictionary rows have a ring of their own (freed by the Gram tile; coefficients
-// and norms stay until the users' product), even and odd chunks have their own
-// eight epilogue warps, and the users' product follows two Gram tiles behind.
-constexpr int kUsers2 = 16; // UMMA N of the users' product
-constexpr int kN2 = 128;    // dictionary rows per chunk: tensor memory holds two Gram buffers and the users' 16 columns
+// Gram tiles (0.33 ms).  With data tile, kernel values and norms in shared memory
+// the products, stores and broadcasts took 1900 cycles a chunk against 1024 of
+// exponentials; with the kernel values in tensor memory the second UMMA (16
+// columns wide, between two Gram tiles) held the tensor pipe for as long as the
+// Gram tile.  So the data tile (converted from the packed rows) is a
+// tensor-memory operand, and the second product is made of warp-level MMAs: an
+// accumulator loaded in the 16x256b shape, exponentiated and converted in place
+// is their operand fragment, with no store, barrier or second pass.  Even and odd
+// chunks have their own eight epilogue warps; three Gram buffers.
+constexpr int kUsers2 = 16; // users of the second product
+constexpr int kN2 = 128;    // dictionary rows per chunk
 constexpr int kStages2 = 4; // chunks' rows in flight
 constexpr int kXStages2 = 4; // chunks' coefficients and norms in flight
 constexpr int kEpiWarps2 = 16;
@@ -521,7 +519,7 @@ constexpr int kXd2 = 2 * kN2 + 4; // chunk norms, fix weights, gate
 struct Gram2Args {
     const float* rows;    // data rows (n_samples x Dp, FP32)
     const uint8_t* b_ops; // dictionary chunks (kN2 rows)
-    const uint8_t* w_ops; // per chunk: W, 16 rows x kN2 (K), canonical K-major
+    const uint8_t* w_ops; // per chunk: coefficient fragments (gram_pack_w_kernel)
     const float* dn;      // dictionary norms (Mpad)
     const float* fw;      // fix weights (Mpad)
     const float* gate;    // per chunk: max fw, max fw |ewl2 dn|, 0, 0
@@ -534,8 +532,18 @@ struct Gram2Args {
     unsigned long long wait_ns; // limit of the bounded waits
 };
 
-// Tensor memory columns: two Gram buffers, the users' sums, the data tile and two P buffers (BF16 pairs)
-constexpr uint32_t kTmUsers = 2 * kN2, kTmA = 320, kTmP = 384;
+// Tensor memory columns: three Gram buffers, the data tile (BF16 pairs)
+constexpr int kBufs2 = 3;
+constexpr uint32_t kTmA = kBufs2 * kN2;
+
+// acc (16 rows x 8 users) += a (16 rows x 16 BF16) b (16 x 8 users)
+__device__ __forceinline__ void warp_mma(float (&acc)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 
 // 32 columns (sd: their norms, fix weights kN2 further) of four rows: thread t's columns 8 e + 2 (t % 4) + {0, 1}
 // of rows t / 4 + 8 m, Gram values v as loaded, kernel values as BF16 pairs into p[m / 2][2 e + m % 2].  CHECK:
@@ -570,16 +578,18 @@ __device__ __forceinline__ uint32_t kernel_values(const uint32_t (&v)[2][16], co
     return mask;
 }
 
-// W chunks: element (u, k) = a[u][c kN2 + k] * wG (0 past M and for u >= users)
+// Coefficients a[u][b] * wG as BF16 (0 past M and for u >= users) in the fragment order of warp_mma: 16 bytes per 16
+// dictionary rows and lane t, word j holding rows 8 (j % 2) + 2 (t % 4) + {0, 1} of user 8 (j / 2) + t / 4.
 __global__ void gram_pack_w_kernel(const float* __restrict__ a, size_t a_stride, int users, int M, int n_chunks, float wG,
-                                   uint8_t* __restrict__ w_ops)
+                                   uint32_t* __restrict__ w_ops)
 {
-    const int total = n_chunks * kUsers2 * kN2;
+    const int total = n_chunks * (kN2 / 16) * 128;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-        const int k = idx % kN2, u = idx / kN2 % kUsers2, c = idx / (kN2 * kUsers2);
-        const int b = c * kN2 + k;
-        const float v = (u < users && b < M) ? __fmul_rn(a[size_t(u) * a_stride + b], wG) : 0.f;
-        put_operand<kBF16>(w_ops + size_t(c) * kUsers2 * kN2 * 2, kUsers2, u, k, v);
+        const int j = idx % 4, t = idx / 4 % 32, u = 8 * (j / 2) + t / 4, b = idx / 128 * 16 + 8 * (j % 2) + 2 * (t % 4);
+        const float* const c = a + size_t(u) * a_stride + b;
+        const __nv_bfloat162 v = __floats2bfloat162_rn(u < users && b < M ? __fmul_rn(c[0], wG) : 0.f,
+                                                       u < users && b + 1 < M ? __fmul_rn(c[1], wG) : 0.f);
+        w_ops[idx] = *reinterpret_cast<const uint32_t*>(&v);
     }
 }
 
@@ -590,20 +600,20 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t b_bytes = uint32_t(N) * g.Kp * T::kElem;
     constexpr uint32_t w_bytes = kUsers2 * N * T::kElem;
+    constexpr int kParts = kEpiWarps2 / 4; // warps that share a row: column halves of even and odd chunks
     uint8_t* const sB = smem;                           // [NS] chunk rows
     uint8_t* const sW = sB + size_t(NS) * b_bytes;      // [NX] chunk coefficients
     float* const sD = reinterpret_cast<float*>(sW + size_t(NX) * w_bytes); // [NX][kXd2]
     float* const sxn = sD + NX * kXd2;                  // [kTileM] data norms
-    uint64_t* const bars = reinterpret_cast<uint64_t*>(sxn + kTileM);
+    float* const red = sxn + kTileM;                    // [kParts][kTileM][kUsers2]
+    uint64_t* const bars = reinterpret_cast<uint64_t*>(red + kParts * kTileM * kUsers2);
     uint64_t* const full = bars;             // [NS]
     uint64_t* const empty = full + NS;       // [NS]
     uint64_t* const xfull = empty + NS;      // [NX]
     uint64_t* const xempty = xfull + NX;     // [NX]
-    uint64_t* const tfull = xempty + NX;     // [2]
-    uint64_t* const tempty = tfull + 2;      // [2]
-    uint64_t* const pfull = tempty + 2;      // [2]
-    uint64_t* const pempty = pfull + 2;      // [2]
-    uint64_t* const afull = pempty + 2;      // [1]
+    uint64_t* const tfull = xempty + NX;     // [kBufs2] Gram tile
+    uint64_t* const tempty = tfull + kBufs2; // [kBufs2]
+    uint64_t* const afull = tempty + kBufs2; // [1]
     uint64_t* const done = afull + 1;        // [1] every product of the CTA completed
     uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* const abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -622,13 +632,11 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
         }
         for (int s = 0; s < NX; ++s) {
             mbar_init(&xfull[s], 1);
-            mbar_init(&xempty[s], 1 + kGroup2);
+            mbar_init(&xempty[s], kGroup2);
         }
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < kBufs2; ++s) {
             mbar_init(&tfull[s], 1);
             mbar_init(&tempty[s], kGroup2);
-            mbar_init(&pfull[s], kGroup2);
-            mbar_init(&pempty[s], 1);
         }
         mbar_init(afull, kEpiWarps2);
         mbar_init(done, 1);
@@ -668,41 +676,21 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
             for (int i = max(0, xissued - NX); i < xissued; ++i) mbar_drain(&xfull[i % NX], (i / NX) & 1);
         }
     } else if (warp == kEpiWarps2 + 1) {
-        // ---------------- MMA issuer: Gram tile of chunk i, then the users' product of chunk i - 2 ----------------
+        // ---------------- MMA issuer ----------------
         if (lane == 0 && mbar_wait(afull, 0, abort_flag, g.wait_ns)) {
             const uint32_t idesc = instr_desc<MODE>(kTileM, N);
-            const uint32_t idesc2 = instr_desc<MODE>(kTileM, kUsers2);
-            constexpr uint32_t lbo = kTileM * 16, lbo_w = kUsers2 * 16;
+            constexpr uint32_t lbo = N * 16;
             const int ksteps = g.Kp / T::kStepK;
-            constexpr int ksteps2 = N / T::kStepK;
-            // One thread issues everything: descriptors are built once, a K step or a buffer is an addition to
-            // their address field (units of 16 bytes).  Building them for every product took 100 cycles each,
-            // more than the products.
-            constexpr uint64_t kStep = 2 * lbo / 16, kStepW = 2 * lbo_w / 16;
-            const uint64_t db = smem_desc(sB, lbo, 128), dw = smem_desc(sW, lbo_w, 128);
+            // One thread issues everything: the descriptor is built once, a K step or a stage is an addition to its
+            // address field (units of 16 bytes).  Building one for every product took 100 cycles each, more than
+            // the product.
+            constexpr uint64_t kStep = 2 * lbo / 16;
             constexpr uint32_t kStepA = T::kStepK / 2; // tensor-memory columns of a K step
-            bool ok = true;
-            auto product2 = [&](int j) {
-                const int pb = j & 1, xj = j % NX;
-                if (!mbar_wait(&xfull[xj], (j / NX) & 1, abort_flag, g.wait_ns) ||
-                    !mbar_wait(&pfull[pb], (j >> 1) & 1, abort_flag, g.wait_ns)) {
-                    ok = false;
-                    return;
-                }
-                tc_fence_after();
-                const uint64_t w = dw + uint64_t(xj) * (w_bytes / 16);
-                const uint32_t p = tmem + kTmP + uint32_t(pb * (N / 2));
-                umma_ts<MODE>(tmem + kTmUsers, p, w, idesc2, j > 0 ? 1u : 0u);
-#pragma unroll
-                for (int kk = 1; kk < ksteps2; ++kk)
-                    umma_ts<MODE>(tmem + kTmUsers, p + kk * kStepA, w + kk * kStepW, idesc2, 1u);
-                umma_commit(&pempty[pb]); // kernel-value buffer free once these products completed
-                umma_commit(&xempty[xj]); // the chunk's coefficients too
-            };
-            for (int i = 0; i < nch && ok; ++i) {
-                const int s = i % NS, buf = i & 1;
+            const uint64_t db = smem_desc(sB, lbo, 128);
+            for (int i = 0; i < nch; ++i) {
+                const int s = i % NS, buf = i % kBufs2;
                 if (!mbar_wait(&full[s], (i / NS) & 1, abort_flag, g.wait_ns)) break;
-                if (i >= 2 && !mbar_wait(&tempty[buf], ((i >> 1) - 1) & 1, abort_flag, g.wait_ns)) break;
+                if (i >= kBufs2 && !mbar_wait(&tempty[buf], ((i / kBufs2) - 1) & 1, abort_flag, g.wait_ns)) break;
                 tc_fence_after();
                 const uint64_t b = db + uint64_t(s) * (b_bytes / 16);
                 const uint32_t d = tmem + uint32_t(buf * N);
@@ -712,16 +700,14 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
                     if (kk < ksteps) umma_ts<MODE>(d, tmem + kTmA + kk * kStepA, b + kk * kStep, idesc, 1u);
                 umma_commit(&tfull[buf]); // Gram tile ready for the epilogue
                 umma_commit(&empty[s]);   // the chunk's rows are free
-                if (i >= 2) product2(i - 2);
             }
-            for (int j = max(0, nch - 2); j < nch && ok && !*abort_flag; ++j) product2(j);
         }
         if (lane == 0) {
             umma_commit(done);
             mbar_drain(done, 0);
         }
     } else {
-        // ---------------- epilogue: kernel values of each chunk into P; at the end the users' sums ----------------
+        // ---------------- epilogue: kernel values of each chunk, times the coefficients ----------------
         const int q = warp & 3, group = warp >> 3, half = (warp >> 2 & 1) * (N / 2); // this warp's columns of its chunks
         const uint32_t tlane = tmem + (uint32_t(q * 32) << 16);
         const int row = tile * kTileM + q * 32 + lane; // of this thread's tensor-memory lane
@@ -767,12 +753,17 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
 #pragma unroll
         for (int m = 0; m < 4; ++m) xn[m] = pack2(sxn[r0 + 8 * m], sxn[r0 + 8 * m]);
         const float exn_max = warp_exn_max(g.ewl2, sxn[q * 32 + lane]);
-        bool ok = true;
-        for (int i = group; i < nch; i += 2) { // buffers of the chunk: Gram tile and P number `group`
-            const int x = i % NX, ph = (i >> 1) & 1;
-            ok = mbar_wait(&xfull[x], (i / NX) & 1, abort_flag, g.wait_ns) &&
-                 mbar_wait(&tfull[group], ph, abort_flag, g.wait_ns) &&
-                 (i < 2 || mbar_wait(&pempty[group], ph ^ 1, abort_flag, g.wait_ns));
+        float acc[2][2][4]; // rows 16 m .., users 8 n ..
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[m][n][j] = 0.f;
+        for (int i = group; i < nch; i += 2) {
+            const int x = i % NX, buf = i % kBufs2;
+            bool ok = mbar_wait(&xfull[x], (i / NX) & 1, abort_flag, g.wait_ns) &&
+                 mbar_wait(&tfull[buf], (i / kBufs2) & 1, abort_flag, g.wait_ns);
             ok = __all_sync(0xffffffffu, ok); // (the loads below are warp-wide)
             if (!ok) break;
             tc_fence_after();
@@ -782,13 +773,13 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
 #pragma unroll 1
             for (int col = half; col < half + N / 2; col += 32) {
                 uint32_t v[2][16], p[2][8];
-                tmem_ld_16x32(tlane + uint32_t(group * N + col), v[0]);
-                tmem_ld_16x32(tlane + (16u << 16) + uint32_t(group * N + col), v[1]);
+                tmem_ld_16x32(tlane + uint32_t(buf * N + col), v[0]);
+                tmem_ld_16x32(tlane + (16u << 16) + uint32_t(buf * N + col), v[1]);
                 tmem_ld_wait(v[0], v[1]);
                 if (col != half) { // the accumulators are in registers
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&tempty[group]);
+                    if (lane == 0) mbar_arrive(&tempty[buf]);
                 }
                 if (!check) {
                     kernel_values<false>(v, sd + col + cp, xn, g.ewl2, p);
@@ -813,34 +804,37 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
                                 }
                     }
                 }
-                const uint32_t tp = tlane + kTmP + uint32_t(group * (N / 2) + col / 2);
                 __syncwarp();
-                tmem_st_16x16(tp, p[0]);
-                tmem_st_16x16(tp + (16u << 16), p[1]);
+                const uint4* const w = reinterpret_cast<const uint4*>(sW + size_t(x) * w_bytes) + (col / 16) * 32 + lane;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const uint4 b = w[32 * k];
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        warp_mma(acc[m][0], p[m][4 * k], p[m][4 * k + 1], p[m][4 * k + 2], p[m][4 * k + 3], b.x, b.y);
+                        warp_mma(acc[m][1], p[m][4 * k], p[m][4 * k + 1], p[m][4 * k + 2], p[m][4 * k + 3], b.z, b.w);
+                    }
+                }
             }
-            tmem_st_wait();
-            tc_fence_before(); // P visible to the tensor cores
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&xempty[x]);
-                mbar_arrive(&pfull[group]);
-            }
+            if (lane == 0) mbar_arrive(&xempty[x]);
         }
-        if (warp < 4) {
-            // the first four warps read the users' sums of their 32 lanes (tcgen05.ld is warp-wide: the
-            // whole warp loads, the lanes of rows past the end discard)
-            float acc[kUsers2];
+        // a row's sums from the four warps that share it, in a fixed order
 #pragma unroll
-            for (int u = 0; u < kUsers2; ++u) acc[u] = 0.f;
-            const bool have = ok && nch > 0 && mbar_wait(done, 0, abort_flag, g.wait_ns);
-            if (__all_sync(0xffffffffu, have)) {
-                tc_fence_after();
-                tmem_ld16(tlane + kTmUsers, acc);
-            }
-            if (row < g.n_samples)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-                for (int u = 0; u < kUsers2; ++u)
-                    if (u < g.users) g.part[(size_t(split) * g.users + u) * g.n_samples + row] = acc[u];
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; j += 2)
+                    *reinterpret_cast<float2*>(red + (size_t(warp >> 2) * kTileM + r0 + 16 * m + 4 * j) * kUsers2 + 8 * n +
+                                               cp) = make_float2(acc[m][n][j], acc[m][n][j + 1]);
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps2 * 32) : "memory");
+        for (int u = warp >> 2; u < g.users; u += kParts) {
+            if (row >= g.n_samples) break;
+            float sum = 0.f;
+#pragma unroll
+            for (int k = 0; k < kParts; ++k) sum += red[(size_t(k) * kTileM + q * 32 + lane) * kUsers2 + u];
+            g.part[(size_t(split) * g.users + u) * g.n_samples + row] = sum;
         }
     }
 
@@ -856,7 +850,8 @@ __global__ void __launch_bounds__(kThreads2, 1) gram_detect2_kernel(Gram2Args g)
 size_t gram2_smem(int Kp)
 {
     return size_t(kStages2) * kN2 * Kp * 2 + size_t(kXStages2) * kUsers2 * kN2 * 2 +
-           sizeof(float) * (kXStages2 * kXd2 + kTileM) + (2 * kStages2 + 2 * kXStages2 + 10) * 8 + 16;
+           sizeof(float) * (kXStages2 * kXd2 + kTileM + kEpiWarps2 / 4 * kTileM * kUsers2) +
+           (2 * kStages2 + 2 * kXStages2 + 2 * kBufs2 + 2) * 8 + 16;
 }
 
 template <int MODE, int NU> void launch_gram(const GramArgs& ga, int n_tiles, int splits, size_t smem, cudaStream_t s,
@@ -906,8 +901,8 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
     gram_fix_kernel<MODE><<<n_chunks, 256, 0, s>>>(h->dict_a.p, h->cap, U, M, N, h->cfg.wG, ewl2, gw->dn.p, gw->fw.p,
                                                    gw->gate.p);
     GR_CK(cudaGetLastError());
-    gram_pack_w_kernel<<<std::min(4096, (n_chunks * kUsers2 * N + threads - 1) / threads), threads, 0, s>>>(
-        h->dict_a.p, h->cap, U, M, n_chunks, h->cfg.wG, gw->w_ops.p);
+    gram_pack_w_kernel<<<std::min(4096, (n_chunks * kUsers2 * N / 2 + threads - 1) / threads), threads, 0, s>>>(
+        h->dict_a.p, h->cap, U, M, n_chunks, h->cfg.wG, reinterpret_cast<uint32_t*>(gw->w_ops.p));
     GR_CK(cudaGetLastError());
 
     Gram2Args ga;
