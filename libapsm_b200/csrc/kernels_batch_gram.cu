@@ -36,6 +36,7 @@
 // pair of a chunk (kernel value <= 1) skips the test.
 #include "apsm_batch.cuh"
 #include "apsm_tc.cuh"
+#include "packed_f32.cuh"
 
 #include <algorithm>
 
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(256) batch_gram_pack_b_kernel(const BatchGramJ
     }
 }
 
-// 16 pairs (32 accumulator columns) of one sample: kernel values from the Gram
+// Single-product forms: 16 pairs (32 accumulator columns) of one sample, kernel values from the Gram
 // cross terms, contracted with the pairs' coefficients into the two soft
 // outputs.  CHECK: pairs whose error bound exceeds kFixEps are left out and
 // returned as bits of the mask (pair j -> bit j).
@@ -243,6 +244,30 @@ __device__ __forceinline__ uint32_t epilogue_pairs16(const float* gv, const floa
         }
     }
     return mask;
+}
+
+// Split forms: 16 pairs (32 accumulator columns) of four samples, kernel values
+// from the Gram cross terms, contracted with the pairs' coefficients into the two
+// soft outputs f[m] = (f0, f1) of row t / 4 + 8 m.  Thread t holds (r, m) of pairs
+// 4 e + t % 4 as loaded (tmem_ld_16x32); aw, nb: the chunk data of its first pair.
+__device__ __forceinline__ void epilogue_pairs(const uint32_t (&v)[2][16], const float* aw, const float* nb,
+                                               const float (&exn)[4], float m2, f32x2 (&f)[4])
+{
+    const f32x2 m22 = pack2(m2, m2);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 a = *reinterpret_cast<const float2*>(aw + 8 * e);
+        const f32x2 a0 = pack2(a.x, a.x), a1 = pack2(a.y, a.y);
+        const float en = nb[4 * e];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const uint32_t* const g = v[m >> 1] + 4 * e + 2 * (m & 1);
+            const float es = exn[m] + en, im = __uint_as_float(g[1]);
+            const float2 x = unpack2(fma2(m22, pack2(__uint_as_float(g[0]), im), pack2(es, es)));
+            const float kA = ex2(fminf(x.x, 0.f)), kP = ex2(fminf(x.y, 0.f)), kM = ex2(fminf(fmaf(-m2, im, es), 0.f));
+            f[m] = fma2(a0, pack2(kA, kP), fma2(a1, pack2(kM, kA), f[m]));
+        }
+    }
 }
 
 // kAtm (CN = 64): the sample tile's operand lives in tensor memory, copied there once by the
@@ -347,33 +372,30 @@ __global__ void __launch_bounds__(kThreads, 2)
         // ---------------- MMA issuer ----------------
         if (lane == 0 && nch > 0 && mbar_wait(afull, 0, abort_flag, wait_ns)) {
             const uint32_t idesc = instr_desc<MODE>(kTileM, CN);
-            const uint32_t lbo_a = kTileM * 16, lbo_b = CN * 16;
+            // One thread issues everything: descriptors are built once, a K step, the lo half or a stage is an
+            // addition to their address field (units of 16 bytes).
+            constexpr uint32_t lbo_a = kTileM * 16, lbo_b = CN * 16;
             const int ksteps = jb.Kp / T::kStepK; // 32 bytes of K per UMMA
-            const int lo_off = jb.Kp / T::kChunk; // 16-byte K chunks to the lo half
+            const uint64_t lo_a = uint64_t(jb.Kp / T::kChunk) * (lbo_a / 16), lo_b = uint64_t(jb.Kp / T::kChunk) * (lbo_b / 16);
+            const uint64_t da = smem_desc(sA, lbo_a, 128), db = smem_desc(sB, lbo_b, 128);
             for (int i = 0; i < nch; ++i) {
                 const int s = i % stages, buf = i & 1;
                 if (!mbar_wait(&full[s], (i / stages) & 1, abort_flag, wait_ns)) break;
                 if (i >= 2 && !mbar_wait(&tempty[buf], ((i >> 1) - 1) & 1, abort_flag, wait_ns)) break;
                 tc_fence_after();
-                const uint8_t* b = sB + size_t(s) * b_stride;
                 const uint32_t d = tmem + uint32_t(buf * CN);
-                for (int kk = 0; kk < ksteps; ++kk) {
-                    const uint64_t bh = smem_desc(b + size_t(2 * kk) * lbo_b, lbo_b, 128);
+                uint64_t a = da, b = db + uint64_t(s) * (b_stride / 16);
+                uint32_t ah = tmem + kAcol; // A hi / lo of a K step: T::kStepK tensor-memory columns each
+                for (int kk = 0; kk < ksteps; ++kk, a += 2 * lbo_a / 16, b += 2 * lbo_b / 16, ah += T::kStepK) {
                     if constexpr (ATM) {
-                        // A hi / lo of this K step: T::kStepK tensor-memory columns each
-                        const uint32_t ah = tmem + kAcol + uint32_t(kk * T::kStepK);
-                        const uint64_t bl = smem_desc(b + size_t(lo_off + 2 * kk) * lbo_b, lbo_b, 128);
-                        umma_ts<MODE>(d, ah, bh, idesc, kk > 0 ? 1u : 0u);
-                        umma_ts<MODE>(d, ah, bl, idesc, 1u);
-                        umma_ts<MODE>(d, ah + uint32_t(jb.Kp), bh, idesc, 1u);
+                        umma_ts<MODE>(d, ah, b, idesc, kk > 0 ? 1u : 0u);
+                        umma_ts<MODE>(d, ah, b + lo_b, idesc, 1u);
+                        umma_ts<MODE>(d, ah + uint32_t(jb.Kp), b, idesc, 1u);
                     } else {
-                        const uint64_t ah = smem_desc(sA + size_t(2 * kk) * lbo_a, lbo_a, 128);
-                        umma<MODE>(d, ah, bh, idesc, kk > 0 ? 1u : 0u);
+                        umma<MODE>(d, a, b, idesc, kk > 0 ? 1u : 0u);
                         if constexpr (T::kSplit) {
-                            const uint64_t al = smem_desc(sA + size_t(lo_off + 2 * kk) * lbo_a, lbo_a, 128);
-                            const uint64_t bl = smem_desc(b + size_t(lo_off + 2 * kk) * lbo_b, lbo_b, 128);
-                            umma<MODE>(d, ah, bl, idesc, 1u);
-                            umma<MODE>(d, al, bh, idesc, 1u);
+                            umma<MODE>(d, a, b + lo_b, idesc, 1u);
+                            umma<MODE>(d, a + lo_a, b, idesc, 1u);
                         }
                     }
                 }
@@ -407,75 +429,144 @@ __global__ void __launch_bounds__(kThreads, 2)
             __syncwarp();
             if (lane == 0) mbar_arrive(afull);
         }
-        const int row = tile * kTileM + q * 32 + lane;
-        const bool valid = row < jb.S;
-        const float xn = valid ? jb.nrm_s[row] : 0.f;
-        // exponents in base 2: ew log2(e) (|x|^2 + |y|^2 - 2 r) = exn + eyn + m2 r, the pair norms
-        // pre-scaled in the chunk data; ew <= 0, so clamping the distance at 0 is clamping the
-        // exponent at 0
-        const float exn = jb.ew2 * xn, m2 = -2.f * jb.ew2;
-        // largest |exn| of the warp's samples (gate of the compensated forms)
-        float exn_max = -exn;
-        if constexpr (fix_scale<MODE>() > 0.f) {
+        if constexpr (T::kSplit) {
+            // A thread's rows r0 + 8 m, pairs lane % 4 of each four (tmem_ld_16x32): the pair's norm and coefficients,
+            // read once from shared memory, serve four samples.  With one row per thread these loads and the
+            // exponentials shared the same queue, which held the special function unit at 74 %.  512 detectors,
+            // TF32 split form, 4 / 8 / 16 / 32 antennas: 1094 / 1150 / 1382 / 1482 us before, 1036 / 1091 / 1292 /
+            // 1347 us now (the exponentials alone 774 / 796 / 914 / 674 us, the products at 32 antennas 940 us).
+            // The single-product forms keep one row per thread: their exact recomputations then read the samples
+            // of neighbouring rows together (96 detectors, bf16: 1.57 against 1.91 ms).
+            const int r0 = q * 32 + (lane >> 2), row0 = tile * kTileM + r0, cp = lane & 3;
+            // exponents in base 2: ew log2(e) (|x|^2 + |y|^2 - 2 r) = exn + eyn + m2 r, the pair norms
+            // pre-scaled in the chunk data; ew <= 0, so clamping the distance at 0 is clamping the
+            // exponent at 0
+            const float m2 = -2.f * jb.ew2;
+            float exn[4];
+            f32x2 f[4];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) exn_max = fmaxf(exn_max, __shfl_xor_sync(0xffffffffu, exn_max, o));
-        }
-        float f0 = 0.f, f1 = 0.f;
-        for (int i = 0; i < nch; ++i) {
-            const int j = i % kXRing, buf = i & 1;
-            if (!mbar_wait(&xfull[j], (i / kXRing) & 1, abort_flag, wait_ns)) break;
-            if (!mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, wait_ns)) break;
-            tc_fence_after();
-            const float* xs = sX + size_t(j) * C::kBx;
-            // can any pair of this chunk exceed the bound for a sample of this warp?  (warp-uniform)
-            const bool check = fix_scale<MODE>() > 0.f && fmaf(exn_max, xs[C::kGate], xs[C::kGate + 1]) > 1.f;
+            for (int m = 0; m < 4; ++m) {
+                exn[m] = row0 + 8 * m < jb.S ? jb.ew2 * jb.nrm_s[row0 + 8 * m] : 0.f;
+                f[m] = 0ull;
+            }
+            for (int i = 0; i < nch; ++i) {
+                const int j = i % kXRing, buf = i & 1;
+                const bool ready = mbar_wait(&xfull[j], (i / kXRing) & 1, abort_flag, wait_ns) &&
+                                   mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, wait_ns);
+                if (!__all_sync(0xffffffffu, ready)) break; // (the loads below are warp-wide)
+                tc_fence_after();
+                const float* xs = sX + size_t(j) * C::kBx;
 #pragma unroll 1
-            for (int cb = 0; cb < CN / 2; cb += 32) {
-                const int col = h * (CN / 2) + cb; // 32 columns = 16 pairs
-                float gv[32];
-                tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * CN + col), gv);
-                if (!check) {
-                    epilogue_pairs16<false, CN>(gv, xs, col >> 1, exn, m2, f0, f1);
-                    continue;
+                for (int cb = 0; cb < CN / 2; cb += 32) {
+                    const int col = h * (CN / 2) + cb, p0 = (col >> 1) + cp; // 32 columns = 16 pairs
+                    uint32_t v[2][16];
+                    const uint32_t t = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * CN + col);
+                    tmem_ld_16x32(t, v[0]);
+                    tmem_ld_16x32(t + (16u << 16), v[1]);
+                    tmem_ld_wait(v[0], v[1]);
+                    const float* const aw = xs + C::kAw + 2 * p0;
+                    const float* const nb = xs + C::kNrm + p0;
+                    epilogue_pairs(v, aw, nb, exn, m2, f);
                 }
-                uint32_t mask = epilogue_pairs16<true, CN>(gv, xs, col >> 1, exn, m2, f0, f1);
-                if (!valid) mask = 0u;
-                // flagged pairs: r = Re(y^H x), m = Im(y^H x) in FP32 from the samples themselves
-                while (mask) {
-                    const int j = __ffs(mask) - 1;
-                    mask &= mask - 1u;
-                    const int pj = (col >> 1) + j;
-                    const float2* yb = jb.Yd + size_t(i * C::kPairs + pj) * jb.Np;
-                    float re = 0.f, im = 0.f;
-                    for (int k = 0; k < jb.N; ++k) {
-                        const float2 x = jb.rx[size_t(k) * jb.S + row];
-                        const float2 y = yb[k];
-                        re = fmaf(y.x, x.x, fmaf(y.y, x.y, re));
-                        im = fmaf(y.x, x.y, fmaf(-y.y, x.x, im));
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&tempty[buf]);
+                    mbar_arrive(&xempty[j]);
+                }
+            }
+            // a sample's sums: four lanes (pairs modulo 4; lane % 4 = m keeps row r0 + 8 m), two warps (column halves)
+            float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                float2 t = unpack2(f[m]);
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+                    t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+                }
+                if (cp == m) sum = t;
+            }
+            const int r = r0 + 8 * cp, row = tile * kTileM + r;
+            if (h == 1) red[r] = sum;
+            asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
+            if (h == 0 && row < jb.S) {
+                const float2 o = red[r];
+                const float2 l = jb.lin[row];
+                jb.out[row] = make_float2(l.x + (sum.x + o.x), l.y + (sum.y + o.y));
+            }
+        } else {
+            const int row = tile * kTileM + q * 32 + lane;
+            const bool valid = row < jb.S;
+            const float xn = valid ? jb.nrm_s[row] : 0.f;
+            // exponents in base 2: ew log2(e) (|x|^2 + |y|^2 - 2 r) = exn + eyn + m2 r, the pair norms
+            // pre-scaled in the chunk data; ew <= 0, so clamping the distance at 0 is clamping the
+            // exponent at 0
+            const float exn = jb.ew2 * xn, m2 = -2.f * jb.ew2;
+            // largest |exn| of the warp's samples (gate of the compensated forms)
+            float exn_max = -exn;
+            if constexpr (fix_scale<MODE>() > 0.f) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) exn_max = fmaxf(exn_max, __shfl_xor_sync(0xffffffffu, exn_max, o));
+            }
+            float f0 = 0.f, f1 = 0.f;
+            for (int i = 0; i < nch; ++i) {
+                const int j = i % kXRing, buf = i & 1;
+                const bool ready = mbar_wait(&xfull[j], (i / kXRing) & 1, abort_flag, wait_ns) &&
+                                   mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, wait_ns);
+                if (!__all_sync(0xffffffffu, ready)) break; // (the loads below are warp-wide)
+                tc_fence_after();
+                const float* xs = sX + size_t(j) * C::kBx;
+                // can any pair of this chunk exceed the bound for a sample of this warp?  (warp-uniform)
+                const bool check = fix_scale<MODE>() > 0.f && fmaf(exn_max, xs[C::kGate], xs[C::kGate + 1]) > 1.f;
+#pragma unroll 1
+                for (int cb = 0; cb < CN / 2; cb += 32) {
+                    const int col = h * (CN / 2) + cb; // 32 columns = 16 pairs
+                    float gv[32];
+                    tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * CN + col), gv);
+                    if (!check) {
+                        epilogue_pairs16<false, CN>(gv, xs, col >> 1, exn, m2, f0, f1);
+                        continue;
                     }
-                    const float es = exn + xs[C::kNrm + pj];
-                    const float a0 = xs[C::kAw + 2 * pj], a1 = xs[C::kAw + 2 * pj + 1];
-                    const float kA = ex2(fminf(fmaf(m2, re, es), 0.f));
-                    const float kP = ex2(fminf(fmaf(m2, im, es), 0.f));
-                    const float kM = ex2(fminf(fmaf(-m2, im, es), 0.f));
-                    f0 = fmaf(a0, kA, fmaf(a1, kM, f0));
-                    f1 = fmaf(a0, kP, fmaf(a1, kA, f1));
+                    uint32_t mask = epilogue_pairs16<true, CN>(gv, xs, col >> 1, exn, m2, f0, f1);
+                    if (!valid) mask = 0u;
+                    // flagged pairs: r = Re(y^H x), m = Im(y^H x) in FP32 from the samples themselves
+                    while (mask) {
+                        const int j = __ffs(mask) - 1;
+                        mask &= mask - 1u;
+                        const int pj = (col >> 1) + j;
+                        const float2* yb = jb.Yd + size_t(i * C::kPairs + pj) * jb.Np;
+                        float re = 0.f, im = 0.f;
+                        for (int k = 0; k < jb.N; ++k) {
+                            const float2 x = jb.rx[size_t(k) * jb.S + row];
+                            const float2 y = yb[k];
+                            re = fmaf(y.x, x.x, fmaf(y.y, x.y, re));
+                            im = fmaf(y.x, x.y, fmaf(-y.y, x.x, im));
+                        }
+                        const float es = exn + xs[C::kNrm + pj];
+                        const float a0 = xs[C::kAw + 2 * pj], a1 = xs[C::kAw + 2 * pj + 1];
+                        const float kA = ex2(fminf(fmaf(m2, re, es), 0.f));
+                        const float kP = ex2(fminf(fmaf(m2, im, es), 0.f));
+                        const float kM = ex2(fminf(fmaf(-m2, im, es), 0.f));
+                        f0 = fmaf(a0, kA, fmaf(a1, kM, f0));
+                        f1 = fmaf(a0, kP, fmaf(a1, kA, f1));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&tempty[buf]);
+                    mbar_arrive(&xempty[j]);
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&tempty[buf]);
-                mbar_arrive(&xempty[j]);
+            asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
+            if (h == 1) red[q * 32 + lane] = make_float2(f0, f1);
+            asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
+            if (h == 0 && row < jb.S) {
+                const float2 o = red[q * 32 + lane];
+                const float2 l = jb.lin[row];
+                jb.out[row] = make_float2(l.x + (f0 + o.x), l.y + (f1 + o.y));
             }
-        }
-        asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
-        if (h == 1) red[q * 32 + lane] = make_float2(f0, f1);
-        asm volatile("bar.sync 1, %0;" ::"r"(kEpiWarps * 32) : "memory");
-        if (h == 0 && row < jb.S) {
-            const float2 o = red[q * 32 + lane];
-            const float2 l = jb.lin[row];
-            jb.out[row] = make_float2(l.x + (f0 + o.x), l.y + (f1 + o.y));
         }
     }
 
