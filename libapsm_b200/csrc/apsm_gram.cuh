@@ -6,6 +6,11 @@
 namespace apsm {
 void gram_workspace_free(GramWorkspace* g);
 
+// out[u][s] = wL <w_u, x_s> + the sums part[split][u][s] in order, u < users <= kLinearUsers.
+constexpr int kLinearUsers = 16;
+cudaError_t launch_linear_part(const float* xs, int Dp, int D, const float* w, float wL, const float* part, int splits,
+                               int users, int n_samples, float* out, size_t out_stride, cudaStream_t s);
+
 // TF32 split form with the data tile in tensor memory (kernels_gram_tmem.cu).
 constexpr int kGramTmemChunk = 128; // dictionary rows per chunk
 struct GramTmemArgs {

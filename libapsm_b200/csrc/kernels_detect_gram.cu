@@ -50,7 +50,7 @@ constexpr int kTileM = 128;       // data rows per CTA tile (UMMA M)
 constexpr int kMaxStages = 3;     // dictionary chunk ring (2 where 3 stages do not fit)
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = (kEpiWarps + 2) * 32;
-constexpr int kMaxUsers = 16;
+constexpr int kMaxUsers = kLinearUsers;
 
 struct GramWorkspace {
     DevBuf<uint8_t> a_ops, b_ops, w_ops; // operand tiles in the UMMA canonical K-major layout
@@ -465,7 +465,10 @@ constexpr int kFinPer = kFinSamples / 32;
 constexpr int kFinThreads = 128; // warp: samples lane + 32 k, users 4 warp ..
 constexpr int kFinPitch = kMaxUsers + 4;
 
-size_t finish_smem(int Dp) { return sizeof(float) * (size_t(kFinSamples) * (Dp + 4) + size_t(Dp) * kFinPitch); }
+size_t finish_smem(int Dp) // at most 44032 bytes
+{
+    return sizeof(float) * (size_t(kFinSamples) * (Dp + 4) + size_t(Dp) * kFinPitch);
+}
 
 __global__ void __launch_bounds__(kFinThreads)
     gram_finish_kernel(const float* __restrict__ xs, int Dp, int D, const float* __restrict__ w, float wL,
@@ -532,18 +535,6 @@ __global__ void __launch_bounds__(kFinThreads)
                 for (int sp = 0; sp < splits; ++sp) gsum += part[(size_t(sp) * users + u0 + u) * n_samples + s];
                 out[size_t(u0 + u) * out_stride + s] = fmaf(wL, lin[k][u], gsum);
             }
-}
-
-// above the 48 KB default: opt in (per device, so on every launch)
-cudaError_t launch_finish(const float* xs, int Dp, int D, const float* w, float wL, const float* part, int splits,
-                          int users, int n_samples, float* out, size_t out_stride, cudaStream_t s)
-{
-    const size_t smem = finish_smem(Dp);
-    const cudaError_t e = cudaFuncSetAttribute(gram_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return e;
-    gram_finish_kernel<<<(n_samples + kFinSamples - 1) / kFinSamples, kFinThreads, smem, s>>>(
-        xs, Dp, D, w, wL, part, splits, users, n_samples, out, out_stride);
-    return cudaGetLastError();
 }
 
 // ------------------------------------------------ two-product form (users >= 4) --
@@ -989,7 +980,7 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
     GR_CK(cudaFuncSetAttribute(gram_detect2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     gram_detect2_kernel<<<dim3(n_tiles, splits), kThreads2, smem, s>>>(ga);
     GR_CK(cudaGetLastError());
-    GR_CK(launch_finish(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
+    GR_CK(launch_linear_part(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
     GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
 #undef GR_CK
     return APSM_OK;
@@ -1049,7 +1040,7 @@ apsm_status run_gram_tmem(apsm_detector* h, uint32_t S, float* d_out, cudaStream
     ga.ewl2 = h->model_params().ew * 1.4426950408889634f;
     ga.wait_ns = wait_limit_ns();
     GR_CK(launch_gram_tmem(ga, gw->dn.p, h->dict_a.p, h->cap, M, h->cfg.wG, gw->xd.p, n_tiles, splits, s));
-    GR_CK(launch_finish(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
+    GR_CK(launch_linear_part(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
     GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
 #undef GR_CK
     return APSM_OK;
@@ -1159,13 +1150,22 @@ apsm_status run_gram(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s)
     else if (U <= 8) launch_gram<MODE, 8>(ga, n_tiles, splits, smem, s, &e);
     else launch_gram<MODE, 16>(ga, n_tiles, splits, smem, s, &e);
     if (e != cudaSuccess) return h->cuda_fail(e, "gram_detect_kernel launch");
-    GR_CK(launch_finish(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
+    GR_CK(launch_linear_part(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));
     GR_CK(cudaMemcpyAsync(gw->h_err, gw->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
 #undef GR_CK
     return APSM_OK;
 }
 
 } // namespace
+
+cudaError_t launch_linear_part(const float* xs, int Dp, int D, const float* w, float wL, const float* part, int splits,
+                               int users, int n_samples, float* out, size_t out_stride, cudaStream_t s)
+{
+    gram_finish_kernel<<<(n_samples + kFinSamples - 1) / kFinSamples, kFinThreads, finish_smem(Dp), s>>>(
+        xs, Dp, D, w, wL, part, splits, users, n_samples, out, out_stride);
+    return cudaGetLastError();
+}
+
 } // namespace apsm
 
 using namespace apsm;

@@ -19,8 +19,10 @@
 // (copyWeightMat, cpp/lib/apsm/apsm_noma_detector.cu:321-346).
 #include "apsm_host.hpp"
 #include "apsm_kernels.cuh"
+#include "apsm_gram.cuh"
 #include "apsm_lls.cuh"
 
+#include <algorithm>
 #include <string>
 
 namespace apsm {
@@ -56,91 +58,91 @@ __global__ void __launch_bounds__(kLlsThreads)
         xz[idx] = v;
     }
     __syncthreads();
+    // a thread sums 2 x 2 entries: one conversion to FP64 per product (they bound the kernel), not two
     double* out = part + size_t(blockIdx.x) * D * W;
-    for (int e = threadIdx.x; e < D * W; e += kLlsThreads) {
-        const int i = e / W, j = e % W;
-        double acc = 0.0;
-        if (j >= i)
-            for (int r = 0; r < nr; ++r) acc = fma(double(xz[r * W + i]), double(xz[r * W + j]), acc);
-        out[e] = acc;
+    const int ti = (D + 1) / 2, tj = (W + 1) / 2;
+    for (int e = threadIdx.x; e < ti * tj; e += kLlsThreads) {
+        const int i = 2 * (e / tj), j = 2 * (e % tj);
+        if (j + 1 < i) continue; // below the diagonal: never read
+        const int i1 = min(i + 1, D - 1), j1 = min(j + 1, W - 1);
+        double a00 = 0.0, a01 = 0.0, a10 = 0.0, a11 = 0.0;
+#pragma unroll 4
+        for (int r = 0; r < nr; ++r) {
+            const float* x = xz + r * W;
+            const double p = x[i], q = x[i1], u = x[j], v = x[j1];
+            a00 = fma(p, u, a00);
+            a01 = fma(p, v, a01);
+            a10 = fma(q, u, a10);
+            a11 = fma(q, v, a11);
+        }
+        out[i * W + j] = a00;
+        if (j + 1 < W) out[i * W + j + 1] = a01;
+        if (i + 1 < D) out[(i + 1) * W + j] = a10;
+        if (i + 1 < D && j + 1 < W) out[(i + 1) * W + j + 1] = a11;
     }
 }
 
-// One CTA: G = sum of the blocks' partials (fixed order), G = L L^T, then
-// L L^T w_u = c_u for every user; w[u][d] = w_u[d] / divide_by.
+// One CTA: G = sum of the blocks' partials (fixed order), G = L D L^T, then
+// L D L^T w_u = c_u for every user; w[u][d] = w_u[d] / divide_by.
+// Bound: the chain of D pivots.  The factorization runs on the upper triangle
+// with the right-hand sides as further columns, so L z = c comes with it; there
+// is no square root, one division and one barrier per pivot, and rows are read
+// along the lanes.  The back substitution goes by columns, one warp per user with
+// its solution in registers (a shuffle and a product per step, no sum over
+// lanes).  32 features, 8 users, 32 blocks: 55 us with L L^T, three barriers a
+// pivot and dot products by shuffles, now 25 us.
 __global__ void __launch_bounds__(kSolveThreads)
     lls_solve_kernel(const double* __restrict__ part, int blocks, int D, int users, float divide_by,
                      float* __restrict__ w, int* __restrict__ err)
 {
-    extern __shared__ double g[]; // [D][W]: G (lower triangle filled by symmetry) then the right-hand sides
+    extern __shared__ double g[]; // [D][W]: upper triangle of G, then the right-hand sides
     const int W = D + users;
-    __shared__ int bad;
-    if (threadIdx.x == 0) bad = 0;
-    for (int e = threadIdx.x; e < D * W; e += kSolveThreads) {
-        const int i = e / W, j = e % W;
-        const int src = (j < D && j < i) ? j * W + i : e; // the upper triangle holds G(i, j) = G(j, i)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (int e = threadIdx.x; e < D * W; e += blockDim.x) {
+        if (e % W < e / W) continue;
         double acc = 0.0;
-        for (int b = 0; b < blocks; ++b) acc += part[size_t(b) * D * W + src];
+#pragma unroll 8
+        for (int b = 0; b < blocks; ++b) acc += part[size_t(b) * D * W + e];
         g[e] = acc;
     }
     __syncthreads();
-    // right-looking Cholesky: after step k, column k below the diagonal holds L(., k)
+    // after step k, row k holds d_k L(., k) and, from column D, (L^-1 c)(k)
     for (int k = 0; k < D; ++k) {
-        const double dkk = g[k * W + k];
-        if (!(dkk > 0.0)) {
-            if (threadIdx.x == 0) bad = 1;
-            break; // uniform: every thread reads the same value
+        const double* const gk = g + k * W;
+        if (!(gk[k] > 0.0)) { // uniform: every thread reads the same value
+            if (threadIdx.x == 0) *err = 1;
+            return;
         }
-        const double lkk = sqrt(dkk);
-        __syncthreads(); // every thread read g(k, k)
-        for (int i = k + 1 + threadIdx.x; i < D; i += kSolveThreads) g[i * W + k] /= lkk;
-        if (threadIdx.x == 0) g[k * W + k] = lkk;
-        __syncthreads();
-        // trailing update of the lower triangle: G(i, j) -= L(i, k) L(j, k), k < j <= i
-        const int m = D - k - 1;
-        for (int e = threadIdx.x; e < m * m; e += kSolveThreads) {
-            const int i = k + 1 + e / m, j = k + 1 + e % m;
-            if (j <= i) g[i * W + j] -= g[i * W + k] * g[j * W + k];
+        const double inv = 1.0 / gk[k];
+        for (int i = k + 1 + warp; i < D; i += warps) {
+            const double l = gk[i] * inv;
+            for (int j = i + lane; j < W; j += 32) g[i * W + j] = fma(-l, gk[j], g[i * W + j]);
         }
         __syncthreads();
     }
-    __syncthreads();
-    if (bad) {
-        if (threadIdx.x == 0) *err = 1;
-        return;
+    // D L^T x = z: x_i = z_i / d_i once every later x_j has been taken out of it
+    constexpr int kT = kMaxFeatures / 32;
+    double inv[kT];
+#pragma unroll
+    for (int t = 0; t < kT; ++t) inv[t] = 32 * t + lane < D ? 1.0 / g[(32 * t + lane) * (W + 1)] : 0.0;
+    for (int u = warp; u < users; u += warps) {
+        double x[kT];
+#pragma unroll
+        for (int t = 0; t < kT; ++t) x[t] = 32 * t + lane < D ? g[(32 * t + lane) * W + D + u] * inv[t] : 0.0;
+#pragma unroll
+        for (int t = kT - 1; t >= 0; --t)
+            for (int i = min(D, 32 * (t + 1)) - 1; i >= 32 * t; --i) {
+                const double xi = __shfl_sync(0xffffffffu, x[t], i & 31);
+#pragma unroll
+                for (int v = 0; v <= t; ++v) {
+                    const int j = 32 * v + lane;
+                    if (j < i) x[v] = fma(-(g[j * W + i] * inv[v]), xi, x[v]);
+                }
+            }
+#pragma unroll
+        for (int t = 0; t < kT; ++t)
+            if (32 * t + lane < D) w[size_t(u) * D + 32 * t + lane] = float(x[t] / double(divide_by));
     }
-    // forward (L z = c) then backward (L^T x = z) substitution, one warp per user
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int u = warp; u < users; u += kSolveThreads / 32) {
-        double* c = g + D + u; // column D + u, stride W
-        for (int i = 0; i < D; ++i) {
-            double acc = 0.0;
-            for (int j = lane; j < i; j += 32) acc += g[i * W + j] * c[j * W];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) c[i * W] = (c[i * W] - acc) / g[i * W + i];
-            __syncwarp();
-        }
-        for (int i = D - 1; i >= 0; --i) {
-            double acc = 0.0;
-            for (int j = i + 1 + lane; j < D; j += 32) acc += g[j * W + i] * c[j * W];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) c[i * W] = (c[i * W] - acc) / g[i * W + i];
-            __syncwarp();
-        }
-        for (int d = lane; d < D; d += 32) w[size_t(u) * D + d] = float(c[d * W] / double(divide_by));
-    }
-}
-
-// out[u][s] = sum_d xs[s][d] * w[u][d]
-__global__ void lls_detect_kernel(const float* __restrict__ xs, int ns, int Dp, int D, const float* __restrict__ w,
-                                  int users, float* __restrict__ out, size_t out_stride)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ns * users) return;
-    const int s = i % ns, u = i / ns;
-    float acc = 0.f;
-    for (int d = 0; d < D; ++d) acc = fmaf(xs[size_t(s) * Dp + d], w[size_t(u) * D + d], acc);
-    out[size_t(u) * out_stride + s] = acc;
 }
 
 } // namespace
@@ -180,7 +182,8 @@ apsm_status lls_solve(apsm_detector* h, const float* rows, int n, const float* y
         return APSM_ERR_UNSUPPORTED;
     }
     LL_CK(cudaFuncSetAttribute(lls_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    lls_solve_kernel<<<1, kSolveThreads, smem, s>>>(l->part.p, blocks, D, U, divide_by, l->w.p, l->err.p);
+    // a pivot's barrier and division cost more than its update of a 32-feature triangle: eight warps there
+    lls_solve_kernel<<<1, D <= 32 ? 256 : kSolveThreads, smem, s>>>(l->part.p, blocks, D, U, divide_by, l->w.p, l->err.p);
     LL_CK(cudaGetLastError());
     int bad = 0;
     LL_CK(cudaMemcpyAsync(&bad, l->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -202,10 +205,12 @@ apsm_status lls_detect(apsm_detector* h, int ns, float* d_out, cudaStream_t s)
         return e == cudaSuccess ? APSM_OK : h->cuda_fail(e, "cudaMemsetAsync");
     }
     const int U = int(h->U);
-    lls_detect_kernel<<<(ns * U + 255) / 256, 256, 0, s>>>(h->xs.p, ns, int(h->Dp), int(h->D), h->lls->w.p, U, d_out,
-                                                          size_t(ns));
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? APSM_OK : h->cuda_fail(e, "lls_detect_kernel");
+    cudaError_t e = cudaSuccess;
+    const int D = int(h->D);
+    for (int u = 0; u < U && e == cudaSuccess; u += kLinearUsers) // est = A_data w
+        e = launch_linear_part(h->xs.p, int(h->Dp), D, h->lls->w.p + size_t(u) * D, 1.f, nullptr, 0,
+                               std::min(U - u, kLinearUsers), ns, d_out + size_t(u) * ns, size_t(ns), s);
+    return e == cudaSuccess ? APSM_OK : h->cuda_fail(e, "lls_detect");
 }
 
 const float* lls_weights(apsm_detector* h) { return h->lls ? h->lls->w.p : nullptr; }
