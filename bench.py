@@ -324,7 +324,7 @@ def run_batched(args, rank: int, world: int) -> dict | None:
     sers = [L.symbol_error_rate(e, d.tx_data, d.modulation) for d, e in zip(dets, est_batched)]
     sweep = float(np.median(stage["sweep"]))
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    slots = sms * (shape["sweep_ctas_per_sm"] or 2)
+    slots = sms * (shape["sweep_ctas_per_sm"] or 1)  # a chain of window 80 has an SM to itself
     lat = latency_roofline(pool, L, dets, ids, dev_in, sweep, slots, clk.get("sm_mhz"))
 
     # ---- e2e: host buffers through the C ABI (staging + copies inside) ----

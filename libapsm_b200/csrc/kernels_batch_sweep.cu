@@ -1,6 +1,8 @@
 // Batched APSM training sweep: one CTA per training job, all jobs in one
 // persistent launch (jobs taken in the order given, longest first, from a
-// counter).
+// counter).  It serves the pools that the window sweep (kernels_window_sweep.cu)
+// does not take: sample steps other than 2, startWithFullWindow, windows above
+// 81 pairs, very small or very large dictionaries.
 //
 // Model and step semantics are the reference's (cpp/lib/apsm/apsm_train.cu:
 // 100-166 host step loop, :271-432 kernel; prediction apsm_detect.cu:170-226):

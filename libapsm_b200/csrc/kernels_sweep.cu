@@ -1,4 +1,7 @@
-// APSM training sweep on B200: the whole pilot sequence in one launch.
+// APSM training sweep on B200 in the reference's summation order: the whole
+// pilot sequence in one launch.  It serves the calls that the window sweep
+// (kernels_window_sweep.cu) does not take: normConstraint, a sample step other
+// than 2, windows above 81 pairs, dictionaries too small for its fetch distance.
 //
 // Reference behaviour restated (cpp/lib/apsm/apsm_train.cu:100-166 host loop,
 // :271-432 kernel, cpp/lib/apsm/apsm_detect.cu:170-226 prediction): at each

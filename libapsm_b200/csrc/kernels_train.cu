@@ -13,7 +13,9 @@
 // window row v never changes during the sweep.  gram_columns_kernel computes
 // every value the sweep can touch once (wG * exp(ew * ||x_u - x_v||^2), the
 // reference's float expression and order) into HBM/L2; the users of one cell
-// share it.  The sweep itself is one launch per user: a thread-block cluster
+// share it.  (Most calls train with the window sweep, kernels_window_sweep.cu,
+// over the pair columns of kernels_pair_columns.cu; what follows serves the
+// others.)  The sweep itself is one launch per user: a thread-block cluster
 // whose CTAs split the projection window, keep replicated coefficients in
 // shared memory, exchange the step's corrections through distributed shared
 // memory and meet at one hardware cluster barrier per step (the reference

@@ -25,14 +25,18 @@
 // (4 fma per pair of pairs: 27.6k fma at window 80, 215 cycles on one SM) and
 // the correction chain between them.  The window matrix in shared memory (the
 // form of kernels_batch_sweep.cu) costs 84 KB of shared-memory reads per step,
-// 650 cycles at best and 2300 as measured with everything else beside them; in
-// registers it costs none.  12 warps hold the 84 x 96 slots of a window of 80
-// (21 row pairs per lane, 84 registers), so that one chain has the SM to itself;
-// 4 more warps, one per scheduler, run the corrections between the updates and
-// prepare entering pairs beside them (16 warps: 128 registers a thread, no
-// spills; 15 + 5 warps at 96 registers spilled and took 4500 cycles a step).  The columns arrive by bulk copies several steps ahead:
-// frozen entries in chunks of 1024 pairs, the last qP + 2 entries of a column
-// straight into window-slot order.
+// 650 cycles at best; in registers it costs none.  12 warps hold the 84 x 96
+// slots of a window of 80 (21 pair slots per lane, three floats each), so that
+// one chain has the SM to itself; 4 more warps, one per scheduler, run the
+// corrections between the updates and prepare entering pairs beside them (16
+// warps: 128 registers a thread, no spills; 15 + 5 warps at 96 registers
+// spilled and took 4500 cycles a step).  Kernel columns arrive by bulk copies,
+// groups of up to four columns several steps ahead, in a ring.
+//
+// Measured, before (kernels_sweep.cu for one detector, kernels_batch_sweep.cu for
+// many) and now: 1000 pilots, 8 users, window 80: 3.65 ms, now 0.98; 600 pilots,
+// window 20: 1.8 ms, now 0.57; 512 detectors (563k steps, window 80): 7.09 ms, now
+// 3.95; 64 pilots appended to 16 dictionaries of 2000: 289 us, now 98.
 #include "apsm_batch.cuh"
 #include "packed_f32.cuh"
 #include "apsm_tc.cuh"
@@ -54,8 +58,7 @@ constexpr int kEvictAhead = 4;          // steps that an evicted pair's data is 
 constexpr int kSampleBatch = 8;         // entering pairs per copy group of samples, two groups in flight
 
 // RG compute warps: lane l holds pair slots l, l + 32, .. (C of them) against the TR row slots of
-// its warp, four registers each: (A, Bp) and (Bm, A), the operands of one packed fma per row of the
-// pair.  A warp reads its rows' corrections once for all its columns (a broadcast read costs the
+// its warp, three registers each (A, Bp, Bm).  A warp reads its rows' corrections once for all its columns (a broadcast read costs the
 // shared-memory pipe as much as any other).  BLOCKS: CTAs per SM that the register bound leaves
 // room for.
 template <int C_, int RG_, int TR_, int BLOCKS_> struct Shape {
@@ -86,6 +89,7 @@ template <class S> struct alignas(128) Shared {
     float2 lp[4 * 32];                           // warp kPrepWarp's share of the starts, by te
     float red[S::kRed];                          // [RG][2 kCols] update partials
     float hw[2 * S::kSlots];                     // first predictions
+    float4 low[32];                              // low parts of v (warp kPrepWarp)
     float vs[kMaxFeatures];
     uint64_t cfull[kGroups], xfull[2];           // column and sample groups have arrived
     BatchTrainJob js;
@@ -178,10 +182,6 @@ __device__ __forceinline__ void load_if(float& a, float& p, float& m, uint32_t a
 }
 
 // asynchronous global -> shared copies of a thread (complete at cp_wait)
-__device__ __forceinline__ void cp_async4(void* dst, const void* src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async8(void* dst, const void* src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -638,11 +638,24 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                 return has ? make_float2(x_lane[at], x_lane[at + y_off]) : make_float2(0.f, 0.f);
             };
             const float2 zero = make_float2(0.f, 0.f);
+            // A pair joins v with Kahan's summation (a plain sum over thousands of pairs was the largest error of w:
+            // 0.3-1.4e-6 against 0.1-0.2e-6).
+            // (the low parts wait in shared memory: registers are short here)
+            m.low[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto join = [](float& v, float& l, float p) {
+                const float y = __fadd_rn(p, l), t = __fadd_rn(v, y);
+                l = __fsub_rn(y, __fsub_rn(t, v));
+                v = t;
+            };
             auto join_v = [&](float2 ab, float2 u0, float2 u1) {
-                v0.x = fmaf(ab.x, u0.x, fmaf(ab.y, u0.y, v0.x));
-                v0.y = fmaf(ab.x, u0.y, fmaf(-ab.y, u0.x, v0.y));
-                v1.x = fmaf(ab.x, u1.x, fmaf(ab.y, u1.y, v1.x));
-                v1.y = fmaf(ab.x, u1.y, fmaf(-ab.y, u1.x, v1.y));
+                float4 l = m.low[lane];
+                join(v0.x, l.x, fmaf(ab.x, u0.x, ab.y * u0.y));
+                join(v0.y, l.y, fmaf(ab.x, u0.y, -ab.y * u0.x));
+                if (N > 32) {
+                    join(v1.x, l.z, fmaf(ab.x, u1.x, ab.y * u1.y));
+                    join(v1.y, l.w, fmaf(ab.x, u1.y, -ab.y * u1.x));
+                }
+                m.low[lane] = l;
             };
             // Columns, from their first frozen entry to the pair itself, one after the other around the stream
             // buffer; lane l plans those of the entering steps te = l mod 32 (and their pairs' targets, scales and
