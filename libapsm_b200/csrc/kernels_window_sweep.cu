@@ -34,9 +34,9 @@
 // groups of up to four columns several steps ahead, in a ring.
 //
 // Measured, before (kernels_sweep.cu for one detector, kernels_batch_sweep.cu for
-// many) and now: 1000 pilots, 8 users, window 80: 3.65 ms, now 0.98; 600 pilots,
-// window 20: 1.8 ms, now 0.57; 512 detectors (563k steps, window 80): 7.09 ms, now
-// 3.95; 64 pilots appended to 16 dictionaries of 2000: 289 us, now 98.
+// many) and now: 1000 pilots, 8 users, window 80: 3.65 ms, now 1.03; 600 pilots,
+// window 20: 1.8 ms, now 0.59; 512 detectors (563k steps, window 80): 7.09 ms, now
+// 4.1; 64 pilots appended to 16 dictionaries of 2000: 289 us, now 98.
 #include "apsm_batch.cuh"
 #include "packed_f32.cuh"
 #include "apsm_tc.cuh"
