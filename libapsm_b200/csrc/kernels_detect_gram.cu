@@ -47,7 +47,7 @@
 namespace apsm {
 
 constexpr int kTileM = 128;       // data rows per CTA tile (UMMA M)
-constexpr int kMaxStages = 3;     // dictionary chunk ring (2 where 3 stages do not fit)
+constexpr int kMaxStages = 3;     // dictionary chunk ring
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = (kEpiWarps + 2) * 32;
 constexpr int kMaxUsers = kLinearUsers;
@@ -407,20 +407,12 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect_kernel(GramArgs g)
             // can any entry of this chunk exceed the bound for a row of this warp?  (warp-uniform)
             const float* gate = xs + (2 + g.users) * N;
             const bool check = fix_scale<MODE>() > 0.f && fmaf(exn_max, gate[0], gate[1]) > 1.f;
-            if (half >= 32) {
-                for (int cb = 0; cb < half; cb += 32) {
-                    const int col = h * half + cb;
-                    float gv[32];
-                    tmem_ld32(trow + uint32_t(col), gv);
-                    if (check) fix(epilogue_columns<32, NU, true>(gv, xs + col, N, xn, g.ewl2, g.users, acc), xs, col, c0 + i);
-                    else epilogue_columns<32, NU, false>(gv, xs + col, N, xn, g.ewl2, g.users, acc);
-                }
-            } else { // 32-column chunks: 16 columns per half
-                const int col = h * half;
-                float gv[16];
-                tmem_ld16(trow + uint32_t(col), gv);
-                if (check) fix(epilogue_columns<16, NU, true>(gv, xs + col, N, xn, g.ewl2, g.users, acc), xs, col, c0 + i);
-                else epilogue_columns<16, NU, false>(gv, xs + col, N, xn, g.ewl2, g.users, acc);
+            for (int cb = 0; cb < half; cb += 32) {
+                const int col = h * half + cb;
+                float gv[32];
+                tmem_ld32(trow + uint32_t(col), gv);
+                if (check) fix(epilogue_columns<32, NU, true>(gv, xs + col, N, xn, g.ewl2, g.users, acc), xs, col, c0 + i);
+                else epilogue_columns<32, NU, false>(gv, xs + col, N, xn, g.ewl2, g.users, acc);
             }
             tc_fence_before();
             __syncwarp();
@@ -1065,16 +1057,16 @@ apsm_status run_gram(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s)
     // more accuracy than its time saves)
     if constexpr (MODE == kBF16)
         if (U >= 4 && !h->gram_one_product) return run_gram2(h, S, d_out, s, Kp);
-    // dictionary chunk width and stages: the data tile and the chunk ring within shared memory
-    // (chunks of 256 down to 64 columns in 3 stages, then 32 columns in 3 or 2 stages)
-    int N = 256, stages = kMaxStages;
+    // dictionary chunk width: the data tile and the chunk ring within shared memory (chunks of 256 down
+    // to 64 columns; 64 fit at 128 features of every form that runs here)
+    int N = 256;
+    const int stages = kMaxStages;
     auto smem_for = [&](int n, int st) {
         return size_t(kTileM) * KE * T::kElem + size_t(st) * (size_t(n) * KE * T::kElem + size_t(n) * 4 * (2 + U) + 16) +
                (2 * st + 6) * 8 + 16 + size_t(4 * 32) * U * 4;
     };
     const size_t limit = 220 * 1024;
-    while (N > 32 && smem_for(N, stages) > limit) N /= 2;
-    if (smem_for(N, stages) > limit) stages = 2;
+    while (N > 64 && smem_for(N, stages) > limit) N /= 2;
     if (smem_for(N, stages) > limit) {
         h->last_error = "Gram detection operands do not fit shared memory";
         return APSM_ERR_UNSUPPORTED;
