@@ -523,6 +523,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 for (int cb = 0; cb < CN / 2; cb += 32) {
                     const int col = h * (CN / 2) + cb; // 32 columns = 16 pairs
                     float gv[32];
+                    __syncwarp(); // (lanes recompute different numbers of pairs)
                     tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * CN + col), gv);
                     if (!check) {
                         epilogue_pairs16<false, CN>(gv, xs, col >> 1, exn, m2, f0, f1);

@@ -235,8 +235,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         float4* __restrict__ Kc = jb.Kc;
         for (int i = 0; i < ntile; ++i) {
             const int s = i % kStages, buf = i & 1;
-            if (!mbar_wait(&full[s], (i / kStages) & 1, abort_flag, wait_ns)) break;
-            if (!mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, wait_ns)) break;
+            const bool ready = mbar_wait(&full[s], (i / kStages) & 1, abort_flag, wait_ns) &&
+                               mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, wait_ns);
+            if (!__all_sync(0xffffffffu, ready)) break; // (the loads below are warp-wide)
             tc_fence_after();
             const int b = (t0 + i) * kRowTile + q * 32 + lane; // this lane's row pair
             const float nb = sN[s * kRowTile + q * 32 + lane];
@@ -244,6 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int cb = 0; cb < kColN / 2; cb += 32) {
                 const int col = h * (kColN / 2) + cb; // 32 accumulator columns = 16 column pairs
                 float gv[32];
+                __syncwarp(); // (lanes store different numbers of entries)
                 tmem_ld32(tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * kColN + col), gv);
 #pragma unroll
                 for (int jj = 0; jj < 16; ++jj) {

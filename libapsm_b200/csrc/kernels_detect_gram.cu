@@ -399,8 +399,9 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect_kernel(GramArgs g)
         for (int i = 0; i < nch; ++i) {
             const int s = i % NS, buf = i & 1;
             // the stage's norms / coefficients (bulk copies) and the accumulator
-            if (!mbar_wait(&full[s], (i / NS) & 1, abort_flag, g.wait_ns)) break;
-            if (!mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, g.wait_ns)) break;
+            const bool ready = mbar_wait(&full[s], (i / NS) & 1, abort_flag, g.wait_ns) &&
+                               mbar_wait(&tfull[buf], (i >> 1) & 1, abort_flag, g.wait_ns);
+            if (!__all_sync(0xffffffffu, ready)) break; // (the loads below are warp-wide)
             tc_fence_after();
             const float* xs = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(sX) + size_t(s) * x_bytes);
             const uint32_t trow = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * N);
@@ -410,6 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1) gram_detect_kernel(GramArgs g)
             for (int cb = 0; cb < half; cb += 32) {
                 const int col = h * half + cb;
                 float gv[32];
+                __syncwarp(); // (lanes recompute different numbers of entries)
                 tmem_ld32(trow + uint32_t(col), gv);
                 if (check) fix(epilogue_columns<32, NU, true>(gv, xs + col, N, xn, g.ewl2, g.users, acc), xs, col, c0 + i);
                 else epilogue_columns<32, NU, false>(gv, xs + col, N, xn, g.ewl2, g.users, acc);
