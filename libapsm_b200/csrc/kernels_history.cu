@@ -6,12 +6,15 @@
 //
 // The reference runs, per step, two detections and six single-block metric
 // kernels, each followed by a host synchronisation.  Here the sweep only
-// stores each step's model (the coefficients of the rows it updated and the
-// linear weights, TrainArgs::snap_a / snap_w) and three kernels evaluate every
-// step at once afterwards:
+// stores each step's model (the coefficients of the rows it updated; the cluster
+// sweeps also the linear weights, TrainArgs::snap_a / snap_w) and these kernels
+// evaluate every step at once afterwards:
 //   history_expand_kernel  per-step coefficients -> dense A[step][row] over the
 //                          universe rows (0 where a row is not in that step's
 //                          dictionary);
+//   history_weight_steps_kernel, history_weight_sum_kernel
+//                          every step's linear weights from those coefficients,
+//                          after the window sweep, which does not store them;
 //   history_eval_kernel    est[step][j] = sum_b A[step][b] wG k(x_b, e_j)
 //                          + wL <w_step, e_j> for 64 steps x 64 evaluation rows
 //                          per block (kernel values computed once per block and
@@ -81,25 +84,27 @@ __global__ void __launch_bounds__(kMaxFeatures) history_weight_steps_kernel(Hist
     const float* A = h.A + (size_t(u) * h.n_steps + t) * h.nU;
     const float* prev = t > 0 ? A - h.nU : h.a0 + size_t(u) * h.a0_stride;
     const int n_prev = t > 0 ? h.nU : h.used_before;
-    float acc = 0.f;
+    double acc = 0.0;
     for (int i = start; i < start + st.n_active; ++i) {
-        const float c = A[i] - (i < n_prev ? prev[i] : 0.f);
-        acc = fmaf(c, h.X[size_t(i) * h.Dp + d], acc);
+        const double c = double(A[i]) - double(i < n_prev ? prev[i] : 0.f);
+        acc = fma(c, double(h.X[size_t(i) * h.Dp + d]), acc);
     }
-    h.snap_w[(size_t(u) * h.n_steps + t) * h.D + d] = acc;
+    h.snap_w[(size_t(u) * h.n_steps + t) * h.D + d] = float(acc);
 }
 
-// ... and their running sums from w0.
+// ... and their running sums from w0, in FP64: no later step corrects a rounding here (the sweep's
+// predictions use its own weights), so a plain FP32 sum drifted with the number of steps -- the EVM of
+// 1500 to 6000 steps was 5e-7 to 1.7e-6 away from 64 bits, now 1.6e-7 to 3.8e-7.
 __global__ void __launch_bounds__(kMaxFeatures) history_weight_sum_kernel(HistoryArgs h)
 {
     const int u = blockIdx.x, d = threadIdx.x;
     if (d >= h.D) return;
-    float w = h.w0[size_t(u) * h.D + d];
+    double w = h.w0[size_t(u) * h.D + d];
     float* p = h.snap_w + size_t(u) * h.n_steps * h.D + d;
 #pragma unroll 8
     for (int t = 0; t < h.n_steps; ++t) {
-        w += p[size_t(t) * h.D];
-        p[size_t(t) * h.D] = w;
+        w += double(p[size_t(t) * h.D]);
+        p[size_t(t) * h.D] = float(w);
     }
 }
 
