@@ -848,7 +848,7 @@ apsm_status apsm_detector::check_train_error()
     int e = 0;
     APSM_CK(cudaMemcpy(&e, train_err.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
-        last_error = "training sweep gave up waiting for its cluster (bounded wait expired)";
+        last_error = "the training sweep gave up waiting on the GPU (bounded wait expired); the trained model is invalid";
         return APSM_ERR_CUDA;
     }
     return APSM_OK;

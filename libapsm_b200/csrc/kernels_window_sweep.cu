@@ -136,15 +136,16 @@ __device__ __forceinline__ float warp_sum_halves(float a, float b, int lane)
     return v;
 }
 
-// Bounded wait for a copy (2 s), kept short: the roles' step loops have to stay in the instruction cache.
-__device__ __forceinline__ bool copy_wait(uint64_t* bar, uint32_t parity, volatile int* abort)
+// Bounded wait for a copy (limit_ns; 0: no wait at all), kept short: the roles' step loops have to stay in the
+// instruction cache.
+__device__ __forceinline__ bool copy_wait(uint64_t* bar, uint32_t parity, volatile int* abort, unsigned long long limit_ns)
 {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_test_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
 #pragma unroll 1
-    while (!mbar_try_wait(bar, parity)) {
+    while (limit_ns == 0 || !mbar_try_wait(bar, parity)) {
         if (*abort) return false;
-        if (global_ns() - t0 > kWaitLimitNs) {
+        if (limit_ns == 0 || global_ns() - t0 > limit_ns) {
             *abort = 1;
             return false;
         }
@@ -245,7 +246,7 @@ struct JobView {
 template <class S>
 __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
     window_sweep_kernel(const BatchTrainJob* __restrict__ jobs, int n_jobs, BatchCommon cm, Layout lay, int* counter,
-                        int* err)
+                        int* err, unsigned long long wait_ns)
 {
     constexpr int C = S::C, RG = S::RG, TR = S::TR, kCols = S::kCols, kSlots = S::kSlots;
     constexpr int kAll = S::kThreads, kSampleGroups = 2;
@@ -720,7 +721,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
             uint32_t seen_c = 0; // groups that have arrived
             auto arrived = [&](int te) {
                 if (te >= T0 || int(seen_c) * batch > te) return;
-                copy_wait(&cfull[(base_c + seen_c) % kGroups], ((base_c + seen_c) / kGroups) & 1u, abort_flag);
+                copy_wait(&cfull[(base_c + seen_c) % kGroups], ((base_c + seen_c) / kGroups) & 1u, abort_flag, wait_ns);
                 ++seen_c;
             };
             // samples, in groups of kSampleBatch entering pairs, one lane each
@@ -738,14 +739,18 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                 ++issued_x;
             };
             uint32_t seen_x = 0;
+            auto samples_arrived = [&]() {
+                copy_wait(&xfull[(base_x + seen_x) % kSampleGroups], ((base_x + seen_x) / kSampleGroups) & 1u, abort_flag,
+                          wait_ns);
+                ++seen_x;
+            };
             // old-pair sums and linear part of the pair entering at step te (called for te = 1, 2, ..)
             auto prepare = [&](int te) {
                 if (te >= T0) return;
                 const int n = hi0 + te - 1;
                 if ((te - 1) % kSampleBatch == 0) {
                     if (te + kSampleBatch < T0) sample_issue(te + kSampleBatch);
-                    copy_wait(&xfull[(base_x + seen_x) % kSampleGroups], ((base_x + seen_x) / kSampleGroups) & 1u, abort_flag);
-                    ++seen_x;
+                    if (te > 1) samples_arrived();
                 }
                 const int at = ((te - 1) & (2 * kSampleBatch - 1)) * 2 * pitch;
                 const float2 x0 = sample(at, has0), x1 = sample(at + 32 * y_m, has1);
@@ -764,7 +769,10 @@ __global__ void __launch_bounds__(S::kThreads, S::kBlocks)
                 lp[(te & 3) * 32 + lane] = make_float2(fmaf(wL, g0, lane == 0 ? ps.x : 0.f), fmaf(wL, g1, lane == 0 ? ps.y : 0.f));
             };
             issue(min(lead, T0 + batch)); // (steps before lead)
-            if (1 < T0) sample_issue(1);
+            if (1 < T0) {
+                sample_issue(1);
+                samples_arrived(); // (right behind its issue: a limit of 0 expires here in every job)
+            }
             arrived(0);
             arrived(1);
             step_sync<1, kAll>();
@@ -927,7 +935,7 @@ cudaError_t launch_window_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCo
         const size_t smem = smem_bytes<S>(l);
         e = cudaFuncSetAttribute(window_sweep_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return true;
-        window_sweep_kernel<S><<<grid, S::kThreads, smem, s>>>(d_jobs, n_jobs, cm, l, d_counter, d_err);
+        window_sweep_kernel<S><<<grid, S::kThreads, smem, s>>>(d_jobs, n_jobs, cm, l, d_counter, d_err, wait_limit_ns());
         e = cudaGetLastError();
         return true;
     });

@@ -56,3 +56,19 @@ def test_pool_tensor_core_columns(expire):
     good = pool.run(jobs)[1].copy()
     expire(lambda: pool.run(jobs))
     np.testing.assert_array_equal(pool.run(jobs)[1], good)
+
+
+@pytest.mark.parametrize("window,pilots,users", [(20, 200, 1), (40, 200, 3), (80, 300, 2), (20, 2800, 2)],
+                         ids=["shape32", "shape64", "shape84", "blocks"])
+def test_training(expire, window, pilots, users):
+    f = synth.generate_frame(72, K=3, N=6, P=pilots, S=100, modulation="QAM16", snr_db=20)
+    det = L.NomaDetectorFactory.build(dict(CFG, windowSize=window, dictionarySize=pilots), 6, num_users=users)
+    det.train(f.rx_train, f.tx_train[:users])
+    good = det.get_state()
+    det.reset_state()
+    assert "training sweep" in expire(lambda: det.train(f.rx_train, f.tx_train[:users]))
+    det.reset_state()
+    det.train(f.rx_train, f.tx_train[:users])
+    again = det.get_state()
+    for k in good:
+        np.testing.assert_array_equal(again[k], good[k])
