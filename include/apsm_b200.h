@@ -294,7 +294,9 @@ apsm_status apsm_pool_reset(apsm_pool* p, uint32_t detector);
 apsm_status apsm_pool_run(apsm_pool* p, uint32_t lane, const apsm_job* jobs, uint32_t n_jobs, int mode);
 /* Waits for the lane's last batch and, for APSM_RUN_HOST_ASYNC, writes its
  * estimates to the caller's buffers; returns the batch's status (an expired
- * bounded wait of a tensor-core kernel: APSM_ERR_CUDA). */
+ * bounded wait of a kernel in any of the lane's batches since the last wait:
+ * APSM_ERR_CUDA, once; the detectors that those batches trained hold an
+ * invalid model until a fresh training). */
 apsm_status apsm_pool_wait(apsm_pool* p, uint32_t lane);
 
 /*

@@ -74,9 +74,8 @@ struct Lane {
     };
     std::vector<CopyOut> pending; // estimates to hand to the caller once the batch finished
     std::vector<void*> retired;   // outgrown page-locked buffers (freed with the pool)
-    int* err = nullptr;           // error flag of the last batch (in the scratch)
-    int* err_host = nullptr;      // its copy in page-locked memory, written by the batch's last copy
-    bool err_copied = false;      // the last batch copies the flag (it has kernels that can set it)
+    int* err_dev = nullptr;       // set by a kernel whose bounded wait expired, cleared when the failure is reported
+    int* err_host = nullptr;      // its copy in page-locked memory, written by a batch's last copy
     bool unfinished = false;      // an APSM_RUN_HOST_ASYNC batch whose finish() has not run yet
     int launches = 0;             // kernels launched by the last batch
     // batch timeline (APSM_POOL_TRACE): stream start, inputs copied, packed, kernel columns, swept,
@@ -422,6 +421,7 @@ apsm_pool::~apsm_pool()
         for (auto& e : l.tr_copy)
             if (e) cudaEventDestroy(e);
         if (l.err_host) cudaFreeHost(l.err_host);
+        if (l.err_dev) cudaFree(l.err_dev);
         if (l.stream) cudaStreamDestroy(l.stream);
     }
     if (sched_stream) {
@@ -1164,9 +1164,8 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
         d->used = 0;
     }
     int* d_counter = reinterpret_cast<int*>(D(off_counter));
-    int* d_err = d_counter + 4;
+    int* d_err = L.err_dev;
 
-    L.err = d_err;
     L.launches = 0;
     if (trace) POOL_CK(cudaEventRecord(L.tr[1], s));
     if (nT > 0) {
@@ -1382,12 +1381,11 @@ apsm_status apsm_pool::run(uint32_t lane_id, const apsm_job* jobs, uint32_t n, i
             for (const auto& q : dp) L.pending.push_back({jobs[q.job].est, q.off_est - est_begin, sizeof(float2) * q.S});
         if (timing) POOL_CK(cudaEventRecord(L.ev[3], s));
     }
-    // the error flag of kernels with bounded waits (tensor-core detection) travels back with the
-    // batch: finish() reads it without a synchronous copy
+    // the error flag of the kernels with bounded waits (tensor-core kernels, the window sweep) travels
+    // back with the batch: finish() reads it without a synchronous copy
     bool any_kc_tc = false;
     for (const auto& t : tp) any_kc_tc = any_kc_tc || t.kc_tc;
-    L.err_copied = nG > 0 || any_kc_tc; // only the tensor-core kernels wait on barriers (bounded, flagging expiry)
-    if (L.err_copied) POOL_CK(cudaMemcpyAsync(L.err_host, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (nG > 0 || any_kc_tc || (nT > 0 && cm.split)) POOL_CK(cudaMemcpyAsync(L.err_host, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (trace) {
         POOL_CK(cudaEventRecord(L.tr[6], s));
         L.traced = true;
@@ -1649,10 +1647,11 @@ apsm_status apsm_pool::check_lane(uint32_t lane_id)
 {
     apsm_pool* p = this;
     Lane& L = lanes[lane_id];
-    if (!L.err || !L.err_host || !L.err_copied) return APSM_OK;
-    const int h = *static_cast<volatile int*>(L.err_host); // copied by the batch before its done event
-    if (h) return fail(APSM_ERR_CUDA, "a bounded wait in a tensor-core kernel expired (results of the batch are invalid)");
-    return APSM_OK;
+    if (!*static_cast<volatile int*>(L.err_host)) return APSM_OK; // copied by the batches before their done events
+    *L.err_host = 0;
+    POOL_CK(cudaMemsetAsync(L.err_dev, 0, sizeof(int), L.stream));
+    return fail(APSM_ERR_CUDA, "a kernel's bounded wait expired: the results of the lane's batches since its last wait "
+                               "are invalid, and the detectors that they trained until a fresh training");
 }
 
 // ==================================================================== ABI ==
@@ -1769,6 +1768,9 @@ extern "C" apsm_status apsm_pool_create(const char* algorithm_json, uint64_t hbm
         if (cudaMallocHost(reinterpret_cast<void**>(&l.err_host), sizeof(int)) != cudaSuccess)
             return failp("cudaMallocHost failed", APSM_ERR_CUDA);
         *l.err_host = 0;
+        if (cudaMalloc(&l.err_dev, sizeof(int)) != cudaSuccess ||
+            cudaMemsetAsync(l.err_dev, 0, sizeof(int), l.stream) != cudaSuccess)
+            return failp("cudaMalloc failed", APSM_ERR_OUT_OF_MEMORY);
         cudaEventRecord(l.done, l.stream);
         cudaEventRecord(l.desc_copied, l.stream);
     }

@@ -72,3 +72,47 @@ def test_training(expire, window, pilots, users):
     again = det.get_state()
     for k in good:
         np.testing.assert_array_equal(again[k], good[k])
+
+
+@pytest.mark.parametrize("antennas,fresh", [(4, True), (16, False)])
+def test_pool_training(expire, antennas, fresh):
+    """FP32 detection beside it: no other kernel of the batch waits."""
+    f = synth.generate_frame(73, K=2, N=antennas, P=150, S=200, modulation="QAM16")
+    g = synth.generate_frame(74, K=2, N=antennas, P=40, S=8, modulation="QAM16")
+    pool = L.DetectorPool(CFG)
+    d = pool.add(antennas)
+    first = L.PoolJob(d, f.rx_train, f.tx_train[0], fresh=True)
+    job = first if fresh else L.PoolJob(d, g.rx_train, g.tx_train[0])
+    detect = L.PoolJob(d, f.rx_data)
+
+    def run():
+        pool.run([first])
+        return pool.run([job, detect])[1].copy()
+
+    good = run()
+    pool.run([first])
+    expire(lambda: pool.run([job, detect]))
+    np.testing.assert_array_equal(run(), good)
+
+
+def test_pool_training_on_device_buffers_reported_after_later_batches(expire):
+    import torch
+
+    f = synth.generate_frame(75, K=2, N=4, P=150, S=200, modulation="QAM16")
+    pool = L.DetectorPool(CFG)
+    d = pool.add(4)
+    rx, tx, data = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (f.rx_train, f.tx_train[0], f.rx_data))
+    est = torch.zeros(f.rx_data.shape[1], dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    train, detect = [L.PoolJob(d, rx, tx, fresh=True)], [L.PoolJob(d, data, est=est)]
+
+    def run():
+        pool.run_device(train)
+        pool.run_device(detect)
+        pool.wait()
+        return est.cpu().numpy().copy()
+
+    good = run()
+    expire(run)
+    pool.wait()  # reported once
+    np.testing.assert_array_equal(run(), good)
