@@ -32,6 +32,16 @@ struct TrainStep {
 
 __host__ __device__ inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
+// Opts a kernel in to dynamic shared memory above the 48 KB default.  The limit belongs to the function on
+// its device, not to a launch or a handle: it is set on every launch, always to the same value (the most that
+// a CTA can have less the kernel's own static shared memory, at most `fixed` bytes), so that host threads with
+// handles of their own never lower it between another thread's call here and its launch.
+constexpr size_t kMaxSmem = 227 * 1024;
+template <class Kernel> inline cudaError_t allow_smem(Kernel* kernel, size_t fixed = 0)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxSmem - fixed));
+}
+
 // Limit (ns) of the bounded barrier waits of the tensor-core kernels and the
 // window sweep, read by their launchers (apsm_set_wait_limit_ns; 2 s unless changed).
 unsigned long long wait_limit_ns();

@@ -319,7 +319,7 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
                     const int nso = (xs + C - 1) / C + 1;
                     const int nsop = int(round_up(uint32_t(nso), 32u));
                     const size_t smem = incremental_smem_bytes(ta.XS, ta.XP, nsop, ta.A_ring);
-                    if (smem > 227 * 1024) continue;
+                    if (smem > kMaxSmem) continue;
                     int mc = 0;
                     cudaError_t e = query_incremental_clusters(C, smem, int(U), &mc);
                     if (e != cudaSuccess) {
@@ -367,7 +367,7 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
                                     kMaxFeatures + 2 * q2 + size_t(nwarps) * 32 + 2 * size_t(ta.XW) + 64) +
                    48;
         };
-        const size_t smem_limit = 227 * 1024;
+        const size_t smem_limit = kMaxSmem;
         struct Choice {
             int C = 0, nwarps = 0, ns = 0, clusters = 0;
             bool staged = false, glob_a = false;

@@ -313,8 +313,7 @@ template <int KC>
 cudaError_t launch(const BatchDetectJob* d_jobs, dim3 grid, int nmax, float wL, float wG, cudaStream_t s)
 {
     const size_t smem = Shape<KC>::smem(nmax);
-    // above the 48 KB default: opt in (per device, so on every launch)
-    const cudaError_t e = cudaFuncSetAttribute(batch_detect_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t e = allow_smem(batch_detect_kernel<KC>, 1024);
     if (e != cudaSuccess) return e;
     batch_detect_kernel<KC><<<grid, kThreads, smem, s>>>(d_jobs, nmax, wL, wG);
     return cudaGetLastError();

@@ -600,13 +600,12 @@ cudaError_t launch_cn(const BatchGramJob* d_jobs, int n_jobs, int max_tiles, int
     if (e != cudaSuccess || total_tiles <= 0) return e;
     // two pipeline stages when that lets two CTAs share an SM, else three if they fit
     // (stages_req 2 or 3 overrides the choice where that many fit)
-    constexpr size_t kSmemMax = 227 * 1024;
-    int stages = (2 * gram_smem<MODE, CN>(Kp, 3) > kSmemMax) ? 2 : 3;
-    if (stages_req == 2 || (stages_req == 3 && gram_smem<MODE, CN>(Kp, 3) <= kSmemMax)) stages = stages_req;
+    int stages = (2 * gram_smem<MODE, CN>(Kp, 3) > kMaxSmem) ? 2 : 3;
+    if (stages_req == 2 || (stages_req == 3 && gram_smem<MODE, CN>(Kp, 3) <= kMaxSmem)) stages = stages_req;
     // every CTA holds 256 TMEM columns: at most two CTAs per SM (512 columns), so
     // shared memory is padded to more than a third of the SM's
     const size_t smem = std::max<size_t>(gram_smem<MODE, CN>(Kp, stages), 80 * 1024);
-    e = cudaFuncSetAttribute(batch_gram_kernel<MODE, CN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    e = allow_smem(batch_gram_kernel<MODE, CN>);
     if (e != cudaSuccess) return e;
     batch_gram_kernel<MODE, CN><<<total_tiles, kThreads, smem, s>>>(d_jobs, n_jobs, d_tile_prefix, Kp, stages, d_err,
                                                                     wait_limit_ns());

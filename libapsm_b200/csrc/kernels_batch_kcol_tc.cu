@@ -304,7 +304,7 @@ cudaError_t launch_batch_kcol_tc(const BatchKcolTcJob* d_jobs, int n_jobs, int m
     // every CTA holds 256 TMEM columns: at most two CTAs per SM (512 columns), so shared memory
     // is padded to more than a third of the SM's
     const size_t smem = std::max<size_t>(kcol_tc_smem(Kpmax), 80 * 1024);
-    e = cudaFuncSetAttribute(kcol_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    e = allow_smem(kcol_tc_kernel);
     if (e != cudaSuccess) return e;
     kcol_tc_kernel<<<total_chunks, kThreads, smem, s>>>(d_jobs, n_jobs, d_chunk_prefix, Kpmax, cm, d_err,
                                                          wait_limit_ns());

@@ -753,10 +753,18 @@ size_t batch_sweep_smem(const BatchCommon& cm)
     return sizeof(float) * f;
 }
 
+// (its static shared memory counts: a configuration that just fits keeps fitting)
+static cudaError_t allow_batch_sweep_smem()
+{
+    cudaFuncAttributes a{};
+    const cudaError_t e = cudaFuncGetAttributes(&a, batch_sweep_kernel);
+    return e == cudaSuccess ? allow_smem(batch_sweep_kernel, a.sharedSizeBytes) : e;
+}
+
 cudaError_t batch_sweep_occupancy(const BatchCommon& cm, int* ctas_per_sm)
 {
     const size_t smem = batch_sweep_smem(cm);
-    cudaError_t e = cudaFuncSetAttribute(batch_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_batch_sweep_smem();
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, batch_sweep_kernel, kThreads, smem);
 }
@@ -767,7 +775,7 @@ cudaError_t launch_batch_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCom
     (void)d_err;
     if (n_jobs <= 0) return cudaSuccess;
     const size_t smem = batch_sweep_smem(cm);
-    cudaError_t e = cudaFuncSetAttribute(batch_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_batch_sweep_smem();
     if (e != cudaSuccess) return e;
     batch_sweep_kernel<<<grid, kThreads, smem, s>>>(d_jobs, n_jobs, cm, d_counter);
     return cudaGetLastError();

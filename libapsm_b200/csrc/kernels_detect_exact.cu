@@ -287,10 +287,7 @@ template <int FC, int W, int KU> cudaError_t launch_shape(const DetectArgs& args
 {
     using S = Shape<FC, W, KU>;
     const size_t smem = S::smem(args.Dp);
-    // above the 48 KB default: opt in (per device, so on every launch)
-    if (const cudaError_t e = cudaFuncSetAttribute(detect_exact_kernel<FC, W, KU>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        e != cudaSuccess)
+    if (const cudaError_t e = allow_smem(detect_exact_kernel<FC, W, KU>); e != cudaSuccess)
         return e; // the error stays for the caller's cudaGetLastError
     const int grid = (args.n_samples + S::kSamples - 1) / S::kSamples;
     detect_exact_kernel<FC, W, KU><<<grid, W * 32, smem, stream>>>(args);

@@ -902,7 +902,7 @@ size_t gram2_smem(int Kp)
 template <int MODE, int NU> void launch_gram(const GramArgs& ga, int n_tiles, int splits, size_t smem, cudaStream_t s,
                                              cudaError_t* e)
 {
-    *e = cudaFuncSetAttribute(gram_detect_kernel<MODE, NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    *e = allow_smem(gram_detect_kernel<MODE, NU>);
     if (*e != cudaSuccess) return;
     gram_detect_kernel<MODE, NU><<<dim3(n_tiles, splits), kThreads, smem, s>>>(ga);
     *e = cudaGetLastError();
@@ -971,7 +971,7 @@ apsm_status run_gram2(apsm_detector* h, uint32_t S, float* d_out, cudaStream_t s
     ga.wait_ns = wait_limit_ns();
     // >= 120 KB keeps one CTA per SM: its tensor memory (512 columns) is never contended
     const size_t smem = std::max<size_t>(gram2_smem(Kp) + 1024, 120 * 1024);
-    GR_CK(cudaFuncSetAttribute(gram_detect2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    GR_CK(allow_smem(gram_detect2_kernel));
     gram_detect2_kernel<<<dim3(n_tiles, splits), kThreads2, smem, s>>>(ga);
     GR_CK(cudaGetLastError());
     GR_CK(launch_linear_part(h->xs.p, Dp, D, h->w.p, h->cfg.wL, gw->part.p, splits, U, ns, d_out, size_t(ns), s));

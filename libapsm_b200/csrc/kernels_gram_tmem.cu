@@ -385,7 +385,7 @@ template <int NU> cudaError_t launch(const GramTmemArgs& g, int n_tiles, int spl
                         sizeof(uint64_t) * (2 * kStages + 2 * kXStages + 6) + 16;
     // more than half of an SM's shared memory: one CTA per SM holds all its tensor memory
     const size_t smem = std::max<size_t>(need, 120 * 1024);
-    const cudaError_t e = cudaFuncSetAttribute(gram_tmem_kernel<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t e = allow_smem(gram_tmem_kernel<NU>);
     if (e != cudaSuccess) return e;
     gram_tmem_kernel<NU><<<dim3(n_tiles, splits), kThreads, smem, s>>>(g);
     return cudaGetLastError();

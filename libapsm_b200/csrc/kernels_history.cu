@@ -280,7 +280,7 @@ cudaError_t launch_history(const HistoryArgs& h, cudaStream_t s)
         if (e != cudaSuccess) return e;
     }
     const size_t smem = history_eval_smem(h.D);
-    e = cudaFuncSetAttribute(history_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    e = allow_smem(history_eval_kernel, 1024);
     if (e != cudaSuccess) return e;
     history_eval_kernel<<<dim3(h.n_tiles, (h.n_steps + kSteps - 1) / kSteps, h.users), kThreads, smem, s>>>(h);
     e = cudaGetLastError();

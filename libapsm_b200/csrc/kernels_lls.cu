@@ -176,12 +176,12 @@ apsm_status lls_solve(apsm_detector* h, const float* rows, int n, const float* y
                                                                              row0, U, l->part.p);
     LL_CK(cudaGetLastError());
     const size_t smem = sizeof(double) * size_t(D) * W;
-    if (smem > 227 * 1024) {
+    if (smem > kMaxSmem) {
         h->last_error = "LLS: " + std::to_string(U) + " users with " + std::to_string(D) +
                         " features exceed the solver's shared memory";
         return APSM_ERR_UNSUPPORTED;
     }
-    LL_CK(cudaFuncSetAttribute(lls_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    LL_CK(allow_smem(lls_solve_kernel));
     // a pivot's barrier and division cost more than its update of a 32-feature triangle: eight warps there
     lls_solve_kernel<<<1, D <= 32 ? 256 : kSolveThreads, smem, s>>>(l->part.p, blocks, D, U, divide_by, l->w.p, l->err.p);
     LL_CK(cudaGetLastError());

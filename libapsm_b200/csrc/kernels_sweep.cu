@@ -449,7 +449,7 @@ cudaError_t launch_train_exact(bool staged, int cluster, int threads, size_t sme
                                const TrainArgs& args, int* max_clusters)
 {
     auto kern = sweep_kernel(staged, args.a_glob != nullptr);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     if (cluster > 8) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -477,7 +477,7 @@ cudaError_t query_train_clusters(bool staged, bool glob_a, int cluster, int thre
                                  int* max_clusters)
 {
     auto kern = sweep_kernel(staged, glob_a);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     if (cluster > 8) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

@@ -488,7 +488,7 @@ int incremental_threads() { return kThreads; }
 
 cudaError_t query_incremental_clusters(int cluster, size_t smem, int users, int* max_clusters)
 {
-    cudaError_t e = cudaFuncSetAttribute(train_inc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem(train_inc_kernel);
     if (e != cudaSuccess) return e;
     if (cluster > 8) {
         e = cudaFuncSetAttribute(train_inc_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -518,7 +518,7 @@ size_t incremental_smem_bytes(int XS, int XP, int NSOp, int A_ring)
 cudaError_t launch_train_incremental(int cluster, size_t smem, cudaStream_t stream, const TrainArgs& args,
                                      int* max_clusters)
 {
-    cudaError_t e = cudaFuncSetAttribute(train_inc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem(train_inc_kernel);
     if (e != cudaSuccess) return e;
     if (cluster > 8) {
         e = cudaFuncSetAttribute(train_inc_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

@@ -854,8 +854,6 @@ using Shape32 = Shape<1, 8, 4, 2>;  // up to 32 pair slots
 using Shape64 = Shape<2, 8, 8, 1>;  // up to 64
 using Shape84 = Shape<3, 12, 7, 1>; // up to 84
 
-constexpr size_t kSmemMax = 227 * 1024;
-
 // Buffer sizes: at least three columns of `range` + 1 entries in flight (one read by the step, one
 // by the step ahead, one on its way), up to 8192 entries; a CTA's share of an SM's shared memory
 // where several run on one.
@@ -865,7 +863,7 @@ template <class S> bool layout_for(int range, int pitch, Layout* l)
     for (l->ring = 256; l->ring < range + 16; l->ring *= 2) {}
     for (int blocks = S::kBlocks; blocks >= 1; --blocks)
         for (l->stream = 8192; l->stream >= S::kMatrix && l->stream >= 3 * (range + 1); l->stream /= 2)
-            if (smem_bytes<S>(*l) <= kSmemMax / blocks - 2048) return true;
+            if (smem_bytes<S>(*l) <= kMaxSmem / blocks - 2048) return true;
     return false;
 }
 
@@ -915,7 +913,7 @@ cudaError_t window_sweep_occupancy(const BatchCommon& cm, int range, int* ctas_p
         Layout l;
         if (!layout_for<S>(range, int(round_up(2 * uint32_t(cm.Np), 4)), &l)) return false;
         const size_t smem = smem_bytes<S>(l);
-        e = cudaFuncSetAttribute(window_sweep_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = allow_smem(window_sweep_kernel<S>);
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, window_sweep_kernel<S>, S::kThreads, smem);
         return true;
@@ -933,7 +931,7 @@ cudaError_t launch_window_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCo
         Layout l;
         if (!layout_for<S>(range, int(round_up(2 * uint32_t(cm.Np), 4)), &l)) return false;
         const size_t smem = smem_bytes<S>(l);
-        e = cudaFuncSetAttribute(window_sweep_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = allow_smem(window_sweep_kernel<S>);
         if (e != cudaSuccess) return true;
         window_sweep_kernel<S><<<grid, S::kThreads, smem, s>>>(d_jobs, n_jobs, cm, l, d_counter, d_err, wait_limit_ns());
         e = cudaGetLastError();
