@@ -50,6 +50,7 @@ apsm_detector::~apsm_detector()
     if (ev1) cudaEventDestroy(ev1);
     for (auto& e : stage_ev)
         if (e) cudaEventDestroy(e);
+    for (auto& e : block_ev) cudaEventDestroy(e);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -253,6 +254,7 @@ apsm_status apsm_detector::train(const float2* d_rx, const float2* d_tx, uint32_
         }
         APSM_CK(steps.ensure(h_steps.size()));
         APSM_CK(cudaMemcpyAsync(steps.p, h_steps.data(), sizeof(TrainStep) * h_steps.size(), cudaMemcpyHostToDevice, s));
+        sweep_blocks = 0;
         if (const int form = window_sweep_fits(h_steps, nU)) {
             APSM_CK(train_window(h_steps, nU, mp, hist_nE > 0, form == 2, s));
             goto sweep_done;
@@ -622,7 +624,12 @@ cudaError_t apsm_detector::train_window(const std::vector<TrainStep>& h_steps, u
     e = cudaMemcpyAsync(sweep_jobs.p, jobs.data(), job_bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, sizeof(int) * list.size(), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(train_err.p, 0, sizeof(int), s);
-    if (e == cudaSuccess) e = cudaEventRecord(stage_ev[0], s);
+    // (events around the sweeps alone: apsm_last_kernel_ms)
+    while (blocks && block_ev.size() < 2 * list.size() && e == cudaSuccess) {
+        cudaEvent_t ev = nullptr;
+        e = cudaEventCreate(&ev);
+        if (e == cudaSuccess) block_ev.push_back(ev);
+    }
     for (size_t i = 0; i < list.size() && e == cudaSuccess; ++i) {
         const Block& b = list[i];
         const BatchTrainJob& j = jobs[i * U];
@@ -632,12 +639,15 @@ cudaError_t apsm_detector::train_window(const std::vector<TrainStep>& h_steps, u
             e = launch_old_pair_sums(j.Kc, b.nP, b.n_first, b.nP - b.n_first, capP, std::max(0, b.hi0 - capP), ua.p, nU, int(U), kBlockSplits,
                                      reinterpret_cast<float2*>(sweep_sums.p), s);
         const int range = blocks ? kBlockPairs + 2 * qP : std::min(capP, b.nP);
+        const cudaEvent_t* const mark = blocks ? &block_ev[2 * i] : stage_ev;
+        if (e == cudaSuccess) e = cudaEventRecord(mark[0], s);
         if (e == cudaSuccess)
             e = launch_window_sweep(reinterpret_cast<const BatchTrainJob*>(sweep_jobs.p) + i * U, int(U), cm, range, int(U),
                                     counters + i, train_err.p, s);
+        if (e == cudaSuccess) e = cudaEventRecord(mark[1], s);
     }
-    if (e == cudaSuccess) e = cudaEventRecord(stage_ev[1], s);
-    stage_valid[0] = true;
+    sweep_blocks = blocks ? list.size() : 0;
+    stage_valid[0] = e == cudaSuccess;
     last_train_cluster = 1;
     last_train_staged = false;
     last_train_glob_a = false;
@@ -837,6 +847,16 @@ apsm_status apsm_detector::stage_ms(float* sweep_ms, float* detect_ms)
         if (!out[k]) continue;
         *out[k] = -1.f;
         if (!stage_valid[k]) continue;
+        if (k == 0 && sweep_blocks > 0) {
+            APSM_CK(cudaEventSynchronize(block_ev[2 * sweep_blocks - 1]));
+            *out[k] = 0.f;
+            for (size_t i = 0; i < sweep_blocks; ++i) {
+                float ms = 0.f;
+                APSM_CK(cudaEventElapsedTime(&ms, block_ev[2 * i], block_ev[2 * i + 1]));
+                *out[k] += ms;
+            }
+            continue;
+        }
         APSM_CK(cudaEventSynchronize(stage_ev[2 * k + 1]));
         APSM_CK(cudaEventElapsedTime(out[k], stage_ev[2 * k], stage_ev[2 * k + 1]));
     }

@@ -93,6 +93,8 @@ struct apsm_detector {
     // stage events of the last train / detect call: [sweep start, sweep end, detect start, detect end]
     cudaEvent_t stage_ev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool stage_valid[2] = {false, false};
+    std::vector<cudaEvent_t> block_ev; // training in blocks: start and end of every block's sweep
+    size_t sweep_blocks = 0;           // blocks of the last training call (0: stage_ev holds its sweep)
     std::string last_error;
 
     // persistent model (dictionary rows oldest first, per-user targets and coefficients)
