@@ -22,8 +22,9 @@
 // Bound: FP32 arithmetic (4N + 8 fma per sample and pair) and the special
 // function unit (3 exponentials).  16 jobs of 8064 samples x 1100 pairs: 95 and
 // 94 us at 4 antennas, 539 and 94 us at 32.  Taken, before (one sample per thread against broadcast
-// dictionary entries, scalar arithmetic) and now: 254 -> 207, 388 -> 287,
-// 638 -> 450, 1119 -> 799 us at 4, 8, 16, 32 antennas.
+// dictionary entries, scalar arithmetic) and now: 264 -> 218, 400 -> 304,
+// 655 -> 469, 1134 -> 819 us at 4, 8, 16, 32 antennas (210, 291, 455, 805 us if
+// kernel values below 2^-126 were always dropped).
 //
 // Layout: a lane works on four pairs (lane + 32 r of a tile of 128) for the
 // eight samples of its warp, packed by twos, so 8 + 16 floats of shared memory
@@ -35,6 +36,8 @@
 // beside another's products (one block of eight: 916 us).
 #include "apsm_batch.cuh"
 #include "packed_f32.cuh"
+
+#include <type_traits>
 
 namespace apsm {
 
@@ -53,12 +56,13 @@ template <int N> __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// base-2 exponential on the special function unit, as the training columns take it (results below
-// 2^-126 are zero)
-__device__ __forceinline__ float ex2(float x)
+// Base-2 exponential on the special function unit; results below 2^-126 are zero, or (SMALL) kept as FP32
+// holds them, which takes three more instructions (7 % of the kernel where every exponential takes them).
+template <bool SMALL> __device__ __forceinline__ float ex2(float x)
 {
     float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    if constexpr (SMALL) asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    else asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -153,6 +157,12 @@ __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDe
 #pragma unroll
     for (int h = 0; h < kH; ++h)
         ens[h] = mul2(pack2(ew2, ew2), *reinterpret_cast<const f32x2*>(nrm + warp * kSpw + 2 * h));
+    float ens_min = 0.f;
+#pragma unroll
+    for (int h = 0; h < kH; ++h) {
+        const float2 e = unpack2(ens[h]);
+        ens_min = fminf(ens_min, fminf(e.x, e.y));
+    }
 
     const float* const xw = xs + size_t(warp) * 2 * kSpw * Np;
     const f32x2 ew2_2 = pack2(ew2, ew2), pos = pack2(2.f * ew2, 2.f * ew2), neg = pack2(-2.f * ew2, -2.f * ew2);
@@ -223,24 +233,36 @@ __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDe
         f32x2 f0[kH], f1[kH];
 #pragma unroll
         for (int h = 0; h < kH; ++h) f0[h] = f1[h] = 0ull;
+        auto kernel_sums = [&](auto small) {
+            constexpr bool SMALL = decltype(small)::value;
 #pragma unroll
-        for (int r = 0; r < kR; ++r) {
-            // rows past the dictionary: copied as zeros, with zero coefficients and an exponent <= 0
-            const f32x2 n2 = pack2(nb[r], nb[r]);
-            const f32x2 a0 = pack2(ab[r].x * wG, ab[r].x * wG), a1 = pack2(ab[r].y * wG, ab[r].y * wG);
+            for (int r = 0; r < kR; ++r) {
+                // rows past the dictionary: copied as zeros, with zero coefficients and an exponent <= 0
+                const f32x2 n2 = pack2(nb[r], nb[r]);
+                const f32x2 a0 = pack2(ab[r].x * wG, ab[r].x * wG), a1 = pack2(ab[r].y * wG, ab[r].y * wG);
 #pragma unroll
-            for (int h = 0; h < kH; ++h) {
-                const f32x2 sum = fma2(ew2_2, n2, ens[h]);
-                const float2 qa = unpack2(fma2(neg, re[r][h], sum));
-                const float2 qp = unpack2(fma2(neg, im[r][h], sum)); // K(2b, 2s+1)
-                const float2 qm = unpack2(fma2(pos, im[r][h], sum)); // K(2b+1, 2s)
-                const f32x2 kA = pack2(ex2(fminf(qa.x, 0.f)), ex2(fminf(qa.y, 0.f)));
-                const f32x2 kP = pack2(ex2(fminf(qp.x, 0.f)), ex2(fminf(qp.y, 0.f)));
-                const f32x2 kM = pack2(ex2(fminf(qm.x, 0.f)), ex2(fminf(qm.y, 0.f)));
-                f0[h] = fma2(a0, kA, fma2(a1, kM, f0[h]));
-                f1[h] = fma2(a0, kP, fma2(a1, kA, f1[h]));
+                for (int h = 0; h < kH; ++h) {
+                    const f32x2 sum = fma2(ew2_2, n2, ens[h]);
+                    const float2 qa = unpack2(fma2(neg, re[r][h], sum));
+                    const float2 qp = unpack2(fma2(neg, im[r][h], sum)); // K(2b, 2s+1)
+                    const float2 qm = unpack2(fma2(pos, im[r][h], sum)); // K(2b+1, 2s)
+                    const f32x2 kA = pack2(ex2<SMALL>(fminf(qa.x, 0.f)), ex2<SMALL>(fminf(qa.y, 0.f)));
+                    const f32x2 kP = pack2(ex2<SMALL>(fminf(qp.x, 0.f)), ex2<SMALL>(fminf(qp.y, 0.f)));
+                    const f32x2 kM = pack2(ex2<SMALL>(fminf(qm.x, 0.f)), ex2<SMALL>(fminf(qm.y, 0.f)));
+                    f0[h] = fma2(a0, kA, fma2(a1, kM, f0[h]));
+                    f1[h] = fma2(a0, kP, fma2(a1, kA, f1[h]));
+                }
             }
-        }
+        };
+        // Can a kernel value of this warp and chunk lie below 2^-126?  A squared distance is at most twice the sum
+        // of the squared norms, so not while ew2 (||y_b||^2 + ||y_s||^2) stays above -63 (-62 leaves room for
+        // rounding).  Both branches compute every larger value alike, so the estimates do not depend on what else
+        // is in the warp.
+        float nb_max = 0.f;
+#pragma unroll
+        for (int r = 0; r < kR; ++r) nb_max = fmaxf(nb_max, nb[r]);
+        if (__any_sync(0xffffffffu, fmaf(ew2, nb_max, ens_min) < -62.f)) kernel_sums(std::true_type());
+        else kernel_sums(std::false_type());
         // the lanes' tree; every level halves the values a lane carries: value j = (sample j / 2, component j % 2)
         // ends in lanes 2j, 2j + 1
         float v[2 * kSpw];
