@@ -22,9 +22,10 @@
 // Bound: FP32 arithmetic (4N + 8 fma per sample and pair) and the special
 // function unit (3 exponentials).  16 jobs of 8064 samples x 1100 pairs: 95 and
 // 94 us at 4 antennas, 539 and 94 us at 32.  Taken, before (one sample per thread against broadcast
-// dictionary entries, scalar arithmetic) and now: 264 -> 218, 400 -> 304,
-// 655 -> 469, 1134 -> 819 us at 4, 8, 16, 32 antennas (210, 291, 455, 805 us if
-// kernel values below 2^-126 were always dropped).
+// dictionary entries, scalar arithmetic) and in this form: 254 -> 207, 388 -> 287,
+// 638 -> 450, 1119 -> 799 us at 4, 8, 16, 32 antennas.  Keeping kernel values below
+// 2^-126 where they matter (low_estimates) moves these by +2, +10, +1, -3 us
+// (choosing the exponential for every warp and chunk cost +9, +13, +13, +17).
 //
 // Layout: a lane works on four pairs (lane + 32 r of a tile of 128) for the
 // eight samples of its warp, packed by twos, so 8 + 16 floats of shared memory
@@ -36,8 +37,6 @@
 // beside another's products (one block of eight: 916 us).
 #include "apsm_batch.cuh"
 #include "packed_f32.cuh"
-
-#include <type_traits>
 
 namespace apsm {
 
@@ -57,7 +56,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait()
 }
 
 // Base-2 exponential on the special function unit; results below 2^-126 are zero, or (SMALL) kept as FP32
-// holds them, which takes three more instructions (7 % of the kernel where every exponential takes them).
+// holds them, which takes three more instructions.
 template <bool SMALL> __device__ __forceinline__ float ex2(float x)
 {
     float y;
@@ -81,9 +80,83 @@ template <int KC> struct Shape {
     static constexpr int kPitch = 2 * KC + 4; // floats per tile row: the float4s of eight neighbouring rows cover the banks
     static constexpr size_t smem(int N)
     {
-        return sizeof(float) * (size_t(kStages) * kChunk * kPitch + size_t(2) * kTile * ((N + 1) & ~1) + 3 * kTile);
+        return sizeof(float) * (size_t(kStages) * kChunk * kPitch + size_t(2) * kTile * ((N + 1) & ~1) + kTile);
     }
 };
+
+// The main loop drops kernel values below 2^-126: less than half a rounding of an estimate of kLow or more (n pairs
+// with |a| wG up to 2^36 / n).  A smaller estimate is formed again with every value FP32 holds; models without a linear
+// part have such estimates far from their dictionary, others hardly but for samples of zero.
+constexpr float kLow = 0x1p-64f;
+
+// Component (lane / 2) % 2 of <w, y_s> for the warp's sample lane / 4 (xw: its samples; sample i, antenna k at
+// 4 ((i / 2) Np + k) + i % 2 and two further)
+__device__ __forceinline__ float linear_part(const BatchDetectJob& jb, const float* xw, int Np, int lane)
+{
+    const float* const x = xw + 4 * (lane >> 3) * Np + (lane >> 2 & 1);
+    const int N = jb.N;
+    float l = 0.f;
+    if (lane & 2)
+        for (int k = 0; k < N; ++k) l = fmaf(__ldg(jb.w + k), x[4 * k + 2], fmaf(-__ldg(jb.w + N + k), x[4 * k], l));
+    else
+        for (int k = 0; k < N; ++k) l = fmaf(__ldg(jb.w + k), x[4 * k], fmaf(__ldg(jb.w + N + k), x[4 * k + 2], l));
+    return l;
+}
+
+// The estimates of the warp's samples with a lane in the mask; sums in the order of the main loop.  Out of line, so
+// that it takes no registers from there.
+__device__ __noinline__ void low_estimates(const BatchDetectJob& jb, const float* xs, const float* nrm, float wL,
+                                           float wG, int s0, uint32_t mask)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = jb.N, Np = jb.Np, Mp = jb.Mp;
+    const float ew2 = jb.ew * kLog2e;
+    const float* const xw = xs + 2 * size_t(warp) * kSpw * Np;
+    float g = 0.f; // lanes 4 i + 2 c: component c of sample i
+    for (int c0 = 0; c0 < Mp; c0 += kChunk) {
+        float f[kSpw][2];
+#pragma unroll
+        for (int i = 0; i < kSpw; ++i) f[i][0] = f[i][1] = 0.f;
+#pragma unroll 1
+        for (int b = c0 + lane; b < min(Mp, c0 + kChunk); b += 32) {
+            const float2* const y = jb.Yd + size_t(b) * Np;
+            float re[kSpw], im[kSpw];
+#pragma unroll
+            for (int i = 0; i < kSpw; ++i) re[i] = im[i] = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < N; ++k) {
+                const float2 d = __ldg(y + k);
+#pragma unroll
+                for (int i = 0; i < kSpw; ++i) {
+                    const float* const x = xw + 4 * ((i >> 1) * Np + k) + (i & 1);
+                    re[i] = fmaf(d.x, x[0], fmaf(d.y, x[2], re[i]));
+                    im[i] = fmaf(-d.y, x[0], fmaf(d.x, x[2], im[i]));
+                }
+            }
+            const float a0 = __ldg(jb.a + 2 * b) * wG, a1 = __ldg(jb.a + 2 * b + 1) * wG, nb = __ldg(jb.nrm_d + b);
+#pragma unroll
+            for (int i = 0; i < kSpw; ++i) {
+                const float q = fmaf(ew2, nb, ew2 * nrm[warp * kSpw + i]);
+                const float kA = ex2<true>(fminf(fmaf(-2.f * ew2, re[i], q), 0.f));
+                const float kP = ex2<true>(fminf(fmaf(-2.f * ew2, im[i], q), 0.f));
+                const float kM = ex2<true>(fminf(fmaf(2.f * ew2, im[i], q), 0.f));
+                f[i][0] = fmaf(a0, kA, fmaf(a1, kM, f[i][0]));
+                f[i][1] = fmaf(a0, kP, fmaf(a1, kA, f[i][1]));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kSpw; ++i)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float v = f[i][c];
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == 4 * i + 2 * c) g += v;
+            }
+    }
+    const int s = s0 + warp * kSpw + lane / 4;
+    if (!(lane & 1) && (mask >> (lane & ~3) & 15u))
+        reinterpret_cast<float*>(jb.out + s)[(lane >> 1) & 1] = fmaf(wL, linear_part(jb, xw, Np, lane), g);
+}
 
 template <int KC>
 __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDetectJob* __restrict__ jobs, int nmax,
@@ -110,7 +183,6 @@ __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDe
     float* const tiles = sm;                           // [kStages][kChunk][P]
     float* const xs = tiles + kStages * kChunk * P;    // [kTile / 2][Np] of (re_2i, re_2i+1, im_2i, im_2i+1)
     float* const nrm = xs + 2 * kTile * Np;            // [kTile]
-    float* const fin = nrm + kTile;                    // [kTile][2]
     __shared__ int s_last;
 
     const int nf = (Np + KC - 1) / KC; // copies of a tile
@@ -157,12 +229,6 @@ __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDe
 #pragma unroll
     for (int h = 0; h < kH; ++h)
         ens[h] = mul2(pack2(ew2, ew2), *reinterpret_cast<const f32x2*>(nrm + warp * kSpw + 2 * h));
-    float ens_min = 0.f;
-#pragma unroll
-    for (int h = 0; h < kH; ++h) {
-        const float2 e = unpack2(ens[h]);
-        ens_min = fminf(ens_min, fminf(e.x, e.y));
-    }
 
     const float* const xw = xs + size_t(warp) * 2 * kSpw * Np;
     const f32x2 ew2_2 = pack2(ew2, ew2), pos = pack2(2.f * ew2, 2.f * ew2), neg = pack2(-2.f * ew2, -2.f * ew2);
@@ -233,36 +299,24 @@ __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDe
         f32x2 f0[kH], f1[kH];
 #pragma unroll
         for (int h = 0; h < kH; ++h) f0[h] = f1[h] = 0ull;
-        auto kernel_sums = [&](auto small) {
-            constexpr bool SMALL = decltype(small)::value;
 #pragma unroll
-            for (int r = 0; r < kR; ++r) {
-                // rows past the dictionary: copied as zeros, with zero coefficients and an exponent <= 0
-                const f32x2 n2 = pack2(nb[r], nb[r]);
-                const f32x2 a0 = pack2(ab[r].x * wG, ab[r].x * wG), a1 = pack2(ab[r].y * wG, ab[r].y * wG);
+        for (int r = 0; r < kR; ++r) {
+            // rows past the dictionary: copied as zeros, with zero coefficients and an exponent <= 0
+            const f32x2 n2 = pack2(nb[r], nb[r]);
+            const f32x2 a0 = pack2(ab[r].x * wG, ab[r].x * wG), a1 = pack2(ab[r].y * wG, ab[r].y * wG);
 #pragma unroll
-                for (int h = 0; h < kH; ++h) {
-                    const f32x2 sum = fma2(ew2_2, n2, ens[h]);
-                    const float2 qa = unpack2(fma2(neg, re[r][h], sum));
-                    const float2 qp = unpack2(fma2(neg, im[r][h], sum)); // K(2b, 2s+1)
-                    const float2 qm = unpack2(fma2(pos, im[r][h], sum)); // K(2b+1, 2s)
-                    const f32x2 kA = pack2(ex2<SMALL>(fminf(qa.x, 0.f)), ex2<SMALL>(fminf(qa.y, 0.f)));
-                    const f32x2 kP = pack2(ex2<SMALL>(fminf(qp.x, 0.f)), ex2<SMALL>(fminf(qp.y, 0.f)));
-                    const f32x2 kM = pack2(ex2<SMALL>(fminf(qm.x, 0.f)), ex2<SMALL>(fminf(qm.y, 0.f)));
-                    f0[h] = fma2(a0, kA, fma2(a1, kM, f0[h]));
-                    f1[h] = fma2(a0, kP, fma2(a1, kA, f1[h]));
-                }
+            for (int h = 0; h < kH; ++h) {
+                const f32x2 sum = fma2(ew2_2, n2, ens[h]);
+                const float2 qa = unpack2(fma2(neg, re[r][h], sum));
+                const float2 qp = unpack2(fma2(neg, im[r][h], sum)); // K(2b, 2s+1)
+                const float2 qm = unpack2(fma2(pos, im[r][h], sum)); // K(2b+1, 2s)
+                const f32x2 kA = pack2(ex2<false>(fminf(qa.x, 0.f)), ex2<false>(fminf(qa.y, 0.f)));
+                const f32x2 kP = pack2(ex2<false>(fminf(qp.x, 0.f)), ex2<false>(fminf(qp.y, 0.f)));
+                const f32x2 kM = pack2(ex2<false>(fminf(qm.x, 0.f)), ex2<false>(fminf(qm.y, 0.f)));
+                f0[h] = fma2(a0, kA, fma2(a1, kM, f0[h]));
+                f1[h] = fma2(a0, kP, fma2(a1, kA, f1[h]));
             }
-        };
-        // Can a kernel value of this warp and chunk lie below 2^-126?  A squared distance is at most twice the sum
-        // of the squared norms, so not while ew2 (||y_b||^2 + ||y_s||^2) stays above -63 (-62 leaves room for
-        // rounding).  Both branches compute every larger value alike, so the estimates do not depend on what else
-        // is in the warp.
-        float nb_max = 0.f;
-#pragma unroll
-        for (int r = 0; r < kR; ++r) nb_max = fmaxf(nb_max, nb[r]);
-        if (__any_sync(0xffffffffu, fmaf(ew2, nb_max, ens_min) < -62.f)) kernel_sums(std::true_type());
-        else kernel_sums(std::false_type());
+        }
         // the lanes' tree; every level halves the values a lane carries: value j = (sample j / 2, component j % 2)
         // ends in lanes 2j, 2j + 1
         float v[2 * kSpw];
@@ -303,32 +357,23 @@ __global__ void __launch_bounds__(kThreads, 3) batch_detect_kernel(const BatchDe
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        if (tid < kTile && s0 + tid < S) {
-            float2 g = make_float2(0.f, 0.f);
+    }
+    // every warp finishes its own samples: the lane's value, with the linear part
+    const int s = s0 + warp * kSpw + lane / 4, c = (lane >> 1) & 1;
+    bool low = false;
+    if (s < S) {
+        if (split) {
+            t = 0.f;
 #pragma unroll 8
-            for (int c = 0; c < n_chunks; ++c) {
-                const float2 v = __ldcg(jb.part + size_t(c) * S + s0 + tid);
-                g.x += v.x;
-                g.y += v.y;
-            }
-            *reinterpret_cast<float2*>(fin + 2 * tid) = g;
+            for (int k = 0; k < n_chunks; ++k)
+                t += __ldcg(reinterpret_cast<const float*>(jb.part + size_t(k) * S + s) + c);
         }
-    } else if (!(lane & 1)) {
-        fin[2 * kSpw * warp + (lane >> 1)] = t;
+        const float est = fmaf(wL, linear_part(jb, xw, Np, lane), t);
+        if (!(lane & 1)) reinterpret_cast<float*>(jb.out + s)[c] = est;
+        low = fabsf(est) < kLow;
     }
-    __syncthreads();
-    if (tid < kTile && s0 + tid < S) {
-        const float* const v = xs + 4 * size_t(tid >> 1) * Np + (tid & 1);
-        float l0 = 0.f, l1 = 0.f;
-        for (int k = 0; k < N; ++k) {
-            const float w0 = __ldg(jb.w + k), w1 = __ldg(jb.w + N + k);
-            const float x = v[4 * k], y = v[4 * k + 2];
-            l0 = fmaf(w0, x, fmaf(w1, y, l0));
-            l1 = fmaf(w0, y, fmaf(-w1, x, l1));
-        }
-        const float2 g = *reinterpret_cast<const float2*>(fin + 2 * tid);
-        jb.out[s0 + tid] = make_float2(fmaf(wL, l0, g.x), fmaf(wL, l1, g.y));
-    }
+    const uint32_t mask = __ballot_sync(0xffffffffu, low);
+    if (mask) low_estimates(jb, xs, nrm, wL, wG, s0, mask);
 }
 
 template <int KC>

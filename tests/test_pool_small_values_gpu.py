@@ -42,3 +42,42 @@ def test_kernel_values_below_the_normal_range(oracle_mod, antennas, pilots, symb
     bound = 1e-4 * largest + 4 * 2 * pilots * 2.0**-149
     assert np.max(np.abs(est.real.astype(np.float64) - ref.real)) <= bound
     assert np.max(np.abs(est.imag.astype(np.float64) - ref.imag)) <= bound
+
+
+@pytest.mark.parametrize("symbols", [70, 40000], ids=["split", "unsplit"])
+def test_far_samples_beside_near_ones(oracle_mod, symbols):
+    """Several chunks of the dictionary, spread over blocks or not.  Samples near the dictionary get the bits that
+    they get without the far ones; these are within the 1e-4 of the FP32 form and one step of FP32 of 64 bits, for
+    every coefficient."""
+    antennas, pilots = 4, 300
+    cfg = dict(CFG, dictionarySize=pilots)
+    r = np.random.default_rng(symbols)
+
+    def complex_normal(*shape):
+        return r.standard_normal(shape) + 1j * r.standard_normal(shape)
+
+    rx = (0.01 * complex_normal(antennas, pilots)).astype(np.complex64)
+    tx = (r.choice([-1.0, 1.0], pilots) + 1j * r.choice([-1.0, 1.0], pilots)).astype(np.complex64)
+    data = complex_normal(antennas, symbols)
+    size = 2 * 0.05 * antennas**2
+    data *= np.sqrt(r.uniform(90, 100, symbols) * size / np.sum(np.abs(data) ** 2, axis=0))
+    near = np.arange(symbols) % 3 != 1
+    data[:, near] *= 0.01
+    data = data.astype(np.complex64)
+    pool = DetectorPool(cfg)
+    d = pool.add(antennas)
+    pool.run([PoolJob(d, rx, tx)])
+    est = pool.run([PoolJob(d, data)])[0].copy()
+    alone = pool.run([PoolJob(d, np.ascontiguousarray(data[:, near]))])[0]
+    np.testing.assert_array_equal(est[near], alone)
+    o = oracle_mod.OracleDetector(cfg, antennas, oracle_mod.F64)
+    o.train(rx, tx)
+    far = np.flatnonzero(~near)[:500]
+    ref = o.detect(np.ascontiguousarray(data[:, far]))
+    assert 0.0 < np.max(np.abs(ref)) < 2.0**-126
+    rows = np.concatenate([rx.T, -1j * rx.T]).astype(np.complex128)
+    x = data[:, far].T.astype(np.complex128)
+    total = float(np.sum(np.abs(o.get_state()["a"])))
+    for got, part, rotated in ((est[far].real, ref.real, x), (est[far].imag, ref.imag, -1j * x)):
+        largest = np.exp(-np.min(np.sum(np.abs(rotated[:, None] - rows[None]) ** 2, -1), axis=1) / size)
+        assert np.all(np.abs(got.astype(np.float64) - part) <= total * (1e-4 * largest + 2.0**-149))
