@@ -45,8 +45,9 @@ struct BatchTrainJob {
     const float* y;      // 2 nP targets (row form: Re x, Im x)
     float* a;            // 2 nP coefficients (row form); in: old rows, out: visible rows
     float* w;            // 2N linear weights (in/out)
-    float* r;            // 2N residual weights r = w - sum_{b visible} a_b x_b (in/out, kept with the detector)
-    const float4* Kc;    // kernel columns (A + wL r, Bp + wL m, Bm - wL m, A + wL r), pairs n in [n_first, nP)
+    float* r;            // 2N residual weights (in/out, kept with the detector): r = w - sum a_b x_b over the visible pairs
+                         // (kernels_batch_sweep.cu) or over the window's pairs alone (kernels_window_sweep.cu)
+    const float4* Kc;    // kernel columns (A + wL r, Bp + wL m, Bm - wL m, 0), pairs n in [n_first, nP)
     const TrainStep* steps;
     int n_steps;
     int nP, N, Np, capP; // universe pairs, antennas, row pitch (float2), dictionary capacity in pairs
@@ -219,7 +220,7 @@ cudaError_t batch_sweep_occupancy(const BatchCommon& cm, int* ctas_per_sm);
 cudaError_t launch_batch_sweep(const BatchTrainJob* d_jobs, int n_jobs, BatchCommon cm, int grid, int* d_counter,
                                int* d_err, cudaStream_t s);
 // The sweep with the window matrix in registers (kernels_window_sweep.cu): one pair per step
-// (sp = 1), windows of up to 93 pairs, dictionaries of at least 2 qP + 2 pairs whose frozen part
+// (sp = 1), windows of up to 81 pairs, dictionaries of at least 2 qP + 8 pairs whose frozen part
 // (at most `range` pairs) fits shared memory beside samples of np antennas.
 // The closed form of a schedule with one pair per step (false: not of that form): first visible end and
 // steps per pass, in pairs; full_start: startWithFullWindow.

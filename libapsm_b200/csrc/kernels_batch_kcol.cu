@@ -128,8 +128,7 @@ __global__ void __launch_bounds__(kColRows)
                 const float Bp = wG * ex2_approx(ewl2 * fmaxf(fmaf(-2.f, im[c], sn), 0.f));
                 const float Bm = wG * ex2_approx(ewl2 * fmaxf(fmaf(2.f, im[c], sn), 0.f));
                 const float wc = b >= s_band[c] ? wL : 0.f;
-                const float4 kt = make_float4(fmaf(wc, re[c], A), fmaf(wc, im[c], Bp), fmaf(-wc, im[c], Bm),
-                                              fmaf(wc, re[c], A));
+                const float4 kt = make_float4(fmaf(wc, re[c], A), fmaf(wc, im[c], Bp), fmaf(-wc, im[c], Bm), 0.f);
                 Kc[s_off[c] + b] = kt;
                 if (b >= s_plo[c] && b < s_phi[c]) {
                     // a_2b Kt(2b, .) + a_2b+1 Kt(2b+1, .) for the column pair's two rows

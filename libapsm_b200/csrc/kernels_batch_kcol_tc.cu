@@ -257,8 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const float Bp = wG * ex2(ewl2 * fmaxf(fmaf(-2.f, im, sn), 0.f));
                     const float Bm = wG * ex2(ewl2 * fmaxf(fmaf(2.f, im, sn), 0.f));
                     const float wc = b >= c_band[j] ? wL : 0.f;
-                    const float a = fmaf(wc, re, A);
-                    Kc[c_off[j] + b] = make_float4(a, fmaf(wc, im, Bp), fmaf(-wc, im, Bm), a);
+                    Kc[c_off[j] + b] = make_float4(fmaf(wc, re, A), fmaf(wc, im, Bp), fmaf(-wc, im, Bm), 0.f);
                 }
             }
             tc_fence_before();

@@ -112,7 +112,6 @@ __device__ __forceinline__ void columns_tile(const PairColumnsArgs& g, int b0, i
                     v.y = fmaf(g.wL, li[i][j], v.y);
                     v.z = fmaf(-g.wL, li[i][j], v.z);
                 }
-            v.w = v.x;
             col[b] = v;
         }
     }

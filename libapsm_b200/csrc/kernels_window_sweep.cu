@@ -29,8 +29,8 @@
 // slots of a window of 80 (21 pair slots per lane, three floats each), so that
 // one chain has the SM to itself; 4 more warps, one per scheduler, run the
 // corrections between the updates and prepare entering pairs beside them (16
-// warps: 128 registers a thread, no spills; 15 + 5 warps at 96 registers
-// spilled and took 4500 cycles a step).  Kernel columns arrive by bulk copies,
+// warps: 128 registers a thread and 128 bytes spilled; 15 + 5 warps at 96
+// registers took 4500 cycles a step).  Kernel columns arrive by bulk copies,
 // groups of up to four columns several steps ahead, in a ring.
 //
 // Measured, before (kernels_sweep.cu for one detector, kernels_batch_sweep.cu for
@@ -896,7 +896,7 @@ bool window_schedule(const std::vector<TrainStep>& steps, int qP, int capP, bool
 bool window_sweep_supports(int qP, int sp, int capP, int range, int np)
 {
     // one pair per step; evicted pairs lie before every window pair's combined entries, their
-    // coefficients final when they are fetched kAhead steps early
+    // coefficients final when they are fetched kEvictAhead steps early
     if (sp != 1 || capP < 2 * qP + 2 * kEvictAhead || range < 1) return false;
     return with_shape(qP + 3, [&](auto s) {
         Layout l;
