@@ -53,9 +53,9 @@ sys.path.insert(0, str(ROOT))
 METRIC = "detected symbols/s (batched APSM train + detect, 512 heterogeneous detectors)"
 UNIT = "symbols/s"
 N_DET = 512
-# DRAM bytes per algorithmic byte of the batched sweep (ncu capture of the first
-# 32 detectors: 367.8 MB read + 4.6 MB written for 361.3 MB algorithmic)
-SWEEP_TRAFFIC_PER_ALG_BYTE = (368.360704 + 4.627968) / 361.273728
+# DRAM bytes per algorithmic byte of the window sweep (ncu capture of the first
+# 32 detectors: 361.9 MB read + 5.5 MB written for 361.3 MB algorithmic)
+SWEEP_TRAFFIC_PER_ALG_BYTE = (361.850112 + 5.473536) / 361.273728
 WORKLOAD = {"workload": "512 detectors: N~U{4,8,16,32}, P~U[200,2000], S~U[1000,16000], SNR~U[10,25] dB, "
                         "QPSK/16QAM, window 80, dictionary 2000, fresh train + detect per step",
             "detectors": N_DET, "window": 80, "dictionary": 2000, "detect": "gram_tf32x3 (FP32-accurate)",
@@ -217,14 +217,14 @@ def latency_roofline(pool, L, dets, ids, dev_in, sweep_ms: float, slots: int, sm
     step_us = alone_ms * 1e3 / steps_longest
     total_steps = sum(d.P for d in dets)
     floor_ms = max(steps_longest * step_us, total_steps * step_us / slots) * 1e-3
-    out = {"kernel": "batch_sweep_kernel", "sweep_ms": sweep_ms, "steps_total": total_steps,
+    out = {"kernel": "window_sweep_kernel", "sweep_ms": sweep_ms, "steps_total": total_steps,
            "longest_chain_steps": steps_longest, "slots": slots, "step_us_alone": step_us,
            "chain_floor_ms": steps_longest * step_us * 1e-3,
            "throughput_floor_ms": total_steps * step_us / slots * 1e-3,
            "floor_ms": floor_ms, "frac": floor_ms / sweep_ms,
            "step_us_in_batch": sweep_ms * 1e3 * slots / total_steps,
-           "note": "floor = max(longest chain, all steps / slots) at the step latency of a chain running alone; "
-                   "frac < 1 is what sharing an SM between chains costs"}
+           "note": "floor = max(longest chain, all steps / slots) at the step latency of a chain running alone, "
+                   "which is this kernel's own; frac < 1 is what chains cost one another"}
     if sm_mhz:
         out["cycles_per_step_alone"] = step_us * sm_mhz
         out["cycles_per_step_in_batch"] = out["step_us_in_batch"] * sm_mhz
@@ -400,12 +400,12 @@ def run_batched(args, rank: int, world: int) -> dict | None:
         "training_samples_per_s": pilots / (ms_step * 1e-3),
         "training_samples_per_s_train_stage": pilots / (float(np.median(stage["train"])) * 1e-3),
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "kernel": "batch_sweep_kernel (training sweep, all 512 jobs)",
+        "roofline": {"bound": "hbm", "kernel": "window_sweep_kernel (training sweep, all 512 jobs)",
                      "achieved": achieved, "peak": peak_gbs, "unit": "GB/s", "frac": achieved / peak_gbs,
                      "traffic": alg * SWEEP_TRAFFIC_PER_ALG_BYTE, "algorithmic_bytes_per_launch": alg,
                      "launch_ms": sweep,
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture of the "
-                                       "32-detector case (373.0 MB for 361.3 MB algorithmic), scaled to this "
+                                       "32-detector case (367.3 MB for 361.3 MB algorithmic), scaled to this "
                                        "launch by its algorithmic bytes",
                      "note": "a chain of P dependent steps per detector: bound by step latency (see "
                              "roofline_latency), not HBM; see profiles/",
