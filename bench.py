@@ -469,7 +469,7 @@ def run_plain(steps: int = 5, warmup: int = 3, detect_version: str = "balanced",
     out = {"value": U * S / (ms * 1e-3), "unit": UNIT, "ms_per_step": ms, "ser": ser(est.cpu().numpy()),
            "detect": detect_version,
            "workload": "16QAM K=8 users N=16 P=1000 S=8000 window=80 dictionary=1000, NomaDetector per user "
-                       "(exact FP32 sweep + BALANCED-order detect), all 8 users"}
+                       "(FP32 window sweep + BALANCED-order detect), all 8 users"}
     if not compare:
         det.close()
         return out
@@ -578,7 +578,7 @@ def run_plain_same(dets, dev_in, est_batched) -> dict:
     return {"value": symbols / secs, "unit": UNIT, "seconds": secs, "ser_plain": ser_p, "ser_batched": ser_b,
             "ser_rel_diff": abs(ser_b - ser_p) / ser_p if ser_p else 0.0, "decisions_differing": diff,
             "symbols": symbols,
-            "what": "NomaDetector per detector (exact FP32 sweep + BALANCED-order detect), the 512 frames of the "
+            "what": "NomaDetector per detector (FP32 window sweep + BALANCED-order detect), the 512 frames of the "
                     "batched workload one after the other, device-resident inputs, wall clock with the GPU "
                     "synchronised per detector"}
 
@@ -612,8 +612,8 @@ def model_fp64(state: dict, variance: float, wL: float, wG: float, rx: np.ndarra
 def run_precision_study(reps: int = 3, sample: int = 2048) -> dict:
     """Large detection in every precision: N=64 antennas (128 real features),
     16 16QAM users at 15 dB behind a Rapp PA (p=3), a dictionary of 8192
-    entries filled by 8192 pilots (exact FP32 sweep, all users in one
-    launch), 65536 data symbols detected by one trained model in each form
+    entries filled by 8192 pilots (FP32 window sweep in blocks, all users in one
+    launch each), 65536 data symbols detected by one trained model in each form
     (the model copied into one detector per form).  Two kernel widths: the
     config-0 width (gaussianKernelVariance 0.5, scaled by N^2: a wide kernel,
     the linear part dominates) and the reference's default 0.05 (exponents of

@@ -238,7 +238,7 @@ cudaError_t launch_old_pair_sums(const float4* K, int nP, int n_first, int n_col
                                  size_t a_stride, int users, int splits, float2* out, cudaStream_t s);
 // Jobs of one antenna class (N <= nmax, nmax in {4, 8, 16, 32, 64}).
 // parts: blocks that share one tile of samples, each taking a contiguous run of
-// the job's 64-pair dictionary chunks (1: one block per tile).  Results do not
+// the job's 128-pair dictionary chunks (1: one block per tile).  Results do not
 // depend on parts: every chunk's sum starts from zero and the chunk sums are
 // added in chunk order, by the block itself or by the tile's last block.
 cudaError_t launch_batch_detect(const BatchDetectJob* d_jobs, int n_jobs, int max_tiles, int parts, int nmax, float wL,
